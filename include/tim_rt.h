@@ -103,8 +103,8 @@ typedef struct {
     uint64_t primary_rays, shadow_rays, probe_rays, bounce_rays;
     float kernel_ms;          /* device time of the trace kernels (CUDA events) */
     float total_ms;           /* device time of the whole call incl. copies */
-    /* work counters, filled only with TIM_RT_TRACE_COUNT / TIM_RT_CAM_COUNT:
-     * inner-node fetches (binary: 64-B node, 8-wide: 80-B node), leaf visits,
+    /* work counters, filled only with TIM_RT_TRACE_COUNT / TIM_RT_CAM_COUNT (whose
+     * binary form walks the image's own nodes): inner-node fetches (binary: 64-B node, 8-wide: 80-B node), leaf visits,
      * triangle tests, node-header reloads (8-wide: 32 B when a pending node is popped) */
     uint64_t node_visits, leaf_visits, tri_tests, node_reloads;
     /* camera calls: device time of the primary trace, the secondary-ray
@@ -157,7 +157,11 @@ int tim_rt_measure_l2_bandwidth(int device, uint64_t bytes, int passes, float *g
  * (xyz, xyz, uv per vertex; nrm and uv may be NULL). pc: the scene's PushConstants.
  * The buffers are validated (ranges inside the buffer, node children and leaf
  * offsets in range, vertex indices < num_vertex) before anything is launched;
- * a malformed buffer returns TIM_RT_EINVAL. */
+ * a malformed buffer returns TIM_RT_EINVAL. A context without a memory budget also
+ * builds, on the GPU, the trees its binary-form rays walk (same results): a 4-wide tree
+ * over the image's leaves for any-hit rays and records of child pairs for closest-hit
+ * rays, about 150 B per leaf; a scene that has BLAS instances, or no room for them, is
+ * traced through its own nodes, as in a context with a budget. */
 int tim_rt_upload_bvh(tim_rt_ctx *ctx, const void *bvh_bytes, uint64_t n_bytes, const uint32_t ranges[7][2],
                       const float *pos, const float *nrm, const float *uv, uint32_t max_vertex, uint32_t num_vertex,
                       const tim_rt_push_constants *pc, uint32_t flags, tim_rt_scene_id *out);

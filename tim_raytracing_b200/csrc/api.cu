@@ -262,7 +262,7 @@ int tim_rt_destroy(tim_rt_ctx* c) {
     c->batches.clear();
     for (auto& kv : c->scenes) {
         Scene* s = kv.second.get();
-        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf}) dev_free(c, *b);
+        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
     }
     c->scenes.clear();
     for (DevBuf* b : {&c->rays, &c->hits, &c->nid, &c->bary, &c->counters, &c->cam_out, &c->cam_bounce, &c->cam_nid,
@@ -379,7 +379,7 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
     RawVec<uint32_t> pleaf;
     build_leaf_tris(blob, ranges, pc->numNodes, pos, ptris, pleaf);
     auto fail = [&](int code) {
-        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf}) dev_free(c, *b);
+        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
         return code;
     };
     if ((rc = dev_alloc(c, s->blob, n_bytes))) return fail(rc);
@@ -439,8 +439,12 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
     v.wide_root_is_leaf = wh.root_is_leaf;
     v.pleaf = static_cast<const uint4*>(s->pleaf.ptr);
     v.ptris = static_cast<const float4*>(s->ptris.ptr);
+    uint32_t root_left;   // the root's first child
+    std::memcpy(&root_left, blob + ranges[TIM_RT_RANGE_NODE][0] + 8, 4);
+    root_left &= 0x3FFFFFFFu;
+    if ((rc = build_four(c, s.get(), (uint32_t)(ptris.size() / 12u), root_left))) return fail(rc);
     s->bytes = s->blob.bytes + s->pos.bytes + s->nrm.bytes + s->uv.bytes + s->wnodes.bytes + s->wtris.bytes + s->wnid.bytes +
-               s->pleaf.bytes + s->ptris.bytes;
+               s->pleaf.bytes + s->ptris.bytes + s->nodes4.bytes + s->leaf4.bytes + s->tri_leaf4.bytes + s->pairs.bytes;
     const uint32_t id = c->next_id++;
     c->scenes[id] = std::move(s);
     *out = id;
@@ -473,7 +477,7 @@ int tim_rt_free_scene(tim_rt_ctx* c, tim_rt_scene_id id) {
         return TIM_RT_EINVAL;
     }
     cudaStreamSynchronize(c->stream);
-    for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf}) dev_free(c, *b);
+    for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
     c->scenes.erase(id);
     return TIM_RT_OK;
 }
@@ -528,9 +532,9 @@ int tim_rt_trace_dev(tim_rt_ctx* c, tim_rt_scene_id id, const tim_rt_ray* d_rays
     }
     if (n == 0) return TIM_RT_OK;
     cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : c->stream;
-    uint32_t* ctr = static_cast<uint32_t*>(c->counters.ptr) + kRingBase + (c->ring++ % kRingSize);
+    uint32_t* ctr = static_cast<uint32_t*>(c->counters.ptr) + kRingBase + 2u * (c->ring++ % (kRingSize / 2u));
     uint32_t* err = static_cast<uint32_t*>(c->counters.ptr) + kErrWord;
-    TIMRT_CUDA(cudaMemsetAsync(ctr, 0, 4, st));
+    TIMRT_CUDA(cudaMemsetAsync(ctr, 0, 8, st));
     TIMRT_CUDA(launch_trace_batch(s->view, d_rays, n, mode, d_hit, d_nid, d_bary, ctr, err, st,
                                   cfg_for(c, s, (mode & TIM_RT_TRACE_WIDE) != 0)));
     return TIM_RT_OK;
@@ -564,7 +568,7 @@ int tim_rt_trace(tim_rt_ctx* c, tim_rt_scene_id id, const tim_rt_ray* rays, uint
     if (count) TIMRT_CUDA(cudaMemsetAsync(c->dstats.ptr, 0, 128, c->stream));
     TIMRT_CUDA(cudaEventRecord(c->ev[0], c->stream));
     TIMRT_CUDA(cudaMemcpyAsync(c->rays.ptr, rays, 32ull * n, cudaMemcpyHostToDevice, c->stream));
-    TIMRT_CUDA(cudaMemsetAsync(ctr, 0, 4, c->stream));
+    TIMRT_CUDA(cudaMemsetAsync(ctr, 0, 8, c->stream));
     TIMRT_CUDA(cudaEventRecord(c->ev[1], c->stream));
     TIMRT_CUDA(launch_trace_batch(s->view, static_cast<const tim_rt_ray*>(c->rays.ptr), n, mode,
                                   static_cast<uint32_t*>(c->hits.ptr), leaf_nid ? static_cast<uint32_t*>(c->nid.ptr) : nullptr,

@@ -21,6 +21,8 @@ constexpr uint32_t kNidLeftLeafBit = 0x80000000u;
 constexpr uint32_t kNidRightLeafBit = 0x40000000u;
 constexpr uint32_t kTriBits = 12, kBlasBits = 8, kPrimBits = 8, kLightBits = 4;  // primitive_cpp.glsl:18-21
 constexpr uint32_t kLightSphere = 1u;           // primitive_cpp.glsl:8
+constexpr uint32_t kFourCountShift = 27, kFourFirstMask = (1u << kFourCountShift) - 1u;   // 4-wide tree's leaf references
+constexpr uint32_t kFourBytes = 224u, kPairBytes = 112u;   // a node of the 4-wide tree, a child-pair record
 constexpr int kStackSize = 32;                  // the reference's bitstack is 32 bits wide
 
 // Device view of one uploaded scene (reference layout).
@@ -48,6 +50,14 @@ struct SceneView {
     // positions directly, as the allocation-free entry point does)
     const uint4* pleaf;         // per node: (first triangle, leaf header, leaf-data offset, 0)
     const float4* ptris;        // 3 x float4 per leaf triangle: (p0, vo) (e1, i01) (e2, i2m)
+    // the 4-wide tree of the any-hit rays over the leaves of ptris (trace_any.cuh; null: none)
+    const float4* nodes4;       // 14 x float4 per node
+    const uint4* leaf4;         // 2 per leaf: (E lo.xyz, nid) (E hi.xyz, flag | triangles << 2)
+    const uint32_t* tri_leaf4;  // per triangle of ptris, its leaf in leaf4
+    const float4* pairs;        // the closest-hit rays' records of child pairs, 7 x float4 each (trace_pair.cuh)
+    uint32_t root_pair;         // the root's children
+    uint32_t depth4;            // levels of 4-wide nodes (stack entries needed)
+    float bound4[3];            // largest magnitude of any plane, per axis
 };
 
 struct Ray {

@@ -18,6 +18,8 @@
 #include "common.cuh"
 #include "trace_plain.cuh"
 #include "trace_wide.cuh"
+#include "trace_any.cuh"
+#include "trace_pair.cuh"
 #include "kernels.h"
 #include "../../include/tim_rt.h"
 
@@ -69,6 +71,12 @@ struct finishes { static constexpr bool value = false; };
 template <class P>
 struct finishes<P, decltype((void)P::kFinishes)> { static constexpr bool value = P::kFinishes; };
 
+// Whether a policy traces only the items that keeps() tells of its batch.
+template <class P, class = void>
+struct filters { static constexpr bool value = false; };
+template <class P>
+struct filters<P, decltype((void)P::kFilters)> { static constexpr bool value = P::kFilters; };
+
 struct BatchPolicy {
     const tim_rt_ray* rays;
     uint4* hit;
@@ -99,6 +107,18 @@ struct BatchPolicy {
         }
     }
     __device__ __forceinline__ void skip(uint32_t) const {}
+    __device__ __forceinline__ bool wants_nid() const { return nid != nullptr; }
+    __device__ __forceinline__ bool wants_bary() const { return bary != nullptr; }
+};
+
+// The rays of one kind of a TIM_RT_MODE_PER_RAY batch: the two kinds walk different
+// trees, each in a launch of its own.
+struct KindBatchPolicy : BatchPolicy {
+    static constexpr bool kFilters = true;
+    uint32_t kind;   // TIM_RT_RAY_ANY or 0
+    __device__ __forceinline__ bool keeps(uint32_t i) const {
+        return (__ldg(reinterpret_cast<const uint32_t*>(rays + i) + 7) & TIM_RT_RAY_ANY) == kind;
+    }
 };
 
 // Any-hit rays of a two-level scene (TIM_RT_TRACE_TLAS): traverseTlasFast
@@ -161,14 +181,31 @@ struct CameraPolicy {
         out[2u * pix + 1u] = make_uint4(0u, 0u, 0u, 0u);
         leaf_nid[pix] = 0xFFFFFFFFu;
     }
+    __device__ __forceinline__ bool wants_nid() const { return true; }
+    __device__ __forceinline__ bool wants_bary() const { return false; }
 };
 
-// Secondary rays queued by band and kind (QueueBands); prefix[b * kNumKinds + k] is
-// the first work item of band b's kind k and prefix[n * kNumKinds] the total, so
-// work items run band by band. ray.flags: bit 0 any-hit, bits 8..15 the mask
+// Secondary rays queued by band and kind (QueueBands). Segment e of the work items
+// starts at prefix[e], prefix[n * kNumKinds] being their total. The segments run band
+// by band, or -- closest_last: the two kinds of rays are traced by launches of their
+// own -- the bands' any-hit kinds first and their bounce rays after them, of which a
+// launch traces segments [seg0, seg1). ray.flags: bit 0 any-hit, bits 8..15 the mask
 // bit, bits 16..17 the output (0 shadow mask, 1 probe mask, 2 bounce record).
 // With done / flags (a pipelined camera trace), finished rays are counted per
 // band and flags[b] is set once all of band b's rays are stored.
+__device__ __forceinline__ void segment_of(uint32_t e, uint32_t nb, bool closest_last, uint32_t& band, uint32_t& kind) {
+    if (!closest_last) {
+        band = e / kNumKinds;
+        kind = e - band * kNumKinds;
+    } else if (e < nb * kKindBounce) {
+        band = e / kKindBounce;
+        kind = e - band * kKindBounce;
+    } else {
+        band = e - nb * kKindBounce;
+        kind = kKindBounce;
+    }
+}
+
 struct SecondaryPolicy {
     static constexpr bool kFinishes = true;
     const tim_rt_ray* rays;
@@ -178,16 +215,23 @@ struct SecondaryPolicy {
     uint32_t* out_words;    // tracingData as u32 words (8 per pixel)
     uint4* bounce_out;
     uint32_t* done;         // finished rays per band, or null
+    const uint32_t* band_total;
     volatile uint32_t* flags;
+    uint32_t seg0, seg1;
+    bool closest_last;
 
+    // Work items of the launch: those of its segments.
+    __device__ __forceinline__ uint32_t items() const { return __ldg(prefix + seg1) - __ldg(prefix + seg0); }
     __device__ __forceinline__ bool load(const SceneView&, uint32_t i, TravState& st) const {
-        uint32_t lo = 0, hi = qb.n * kNumKinds;   // largest segment k with prefix[k] <= i
+        i += __ldg(prefix + seg0);
+        uint32_t lo = seg0, hi = seg1;   // largest segment e with prefix[e] <= i
         while (hi - lo > 1u) {
             const uint32_t mid = (lo + hi) >> 1;
             if (__ldg(prefix + mid) <= i) lo = mid;
             else hi = mid;
         }
-        const uint32_t band = lo / kNumKinds, kind = lo - band * kNumKinds;
+        uint32_t band, kind;
+        segment_of(lo, qb.n, closest_last, band, kind);
         const uint32_t slot = qb.base[band] + kind * qb.cap[band] + (i - __ldg(prefix + lo));
         st.slot = slot;
         const float4* rp = reinterpret_cast<const float4*>(rays + slot);
@@ -201,52 +245,98 @@ struct SecondaryPolicy {
         return true;
     }
     // Called by all 32 lanes after a round of stores (`stored`: this lane stored
-    // the ray in queue slot `slot`): one count per band and warp, after each
+    // a ray of pixel `pix`): one count per band and warp, after each
     // storing lane's release fence; the count that completes a band follows every
     // other count of the band in the counter's order, and raises the band's flag
     // after a system-scope fence.
-    __device__ __forceinline__ void finished(bool stored, uint32_t slot) const {
+    __device__ __forceinline__ void finished(bool stored, uint32_t pix) const {
         if (!done) return;
         uint32_t band = 0xFFFFFFFFu;
         if (stored) {
             band = 0;
-            for (uint32_t k = 1; k < qb.n; ++k) band += slot >= qb.base[k] ? 1u : 0u;
+            for (uint32_t k = 1; k < qb.n; ++k) band += pix >= qb.base[k] / kNumKinds ? 1u : 0u;   // base = kNumKinds * W * row
             asm volatile("fence.acq_rel.gpu;" ::: "memory");   // this lane's stores before the warp's count
         }
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, band);
         __syncwarp();
         const uint32_t lane = threadIdx.x & 31u;
         if (stored && lane == (uint32_t)(__ffs(peers) - 1)) {
-            const uint32_t total = __ldg(prefix + (band + 1u) * kNumKinds) - __ldg(prefix + band * kNumKinds);
             const uint32_t cnt = (uint32_t)__popc(peers);
-            if (atomicAdd(done + band, cnt) + cnt == total) {
+            if (atomicAdd(done + band, cnt) + cnt == __ldg(band_total + band)) {
                 __threadfence_system();
                 flags[band] = 1u;
             }
         }
     }
     __device__ __forceinline__ void store(const SceneView&, uint32_t, const TravState& st, float) const {
-        const uint32_t slot = st.slot;
-        const uint32_t fl = __float_as_uint(__ldg(reinterpret_cast<const float*>(rays + slot) + 7));
-        const uint32_t kind = (fl >> 16) & 3u, bit = (fl >> 8) & 0xFFu;
         const uint32_t p = st.slot2;
-        if (kind == 2u) {
+        if (!st.any) {   // a bounce ray
             bounce_out[p] = make_uint4(st.rec0, st.rec1, st.rec2, __float_as_uint(st.t));
         } else if (st.hit) {
+            const uint32_t fl = __float_as_uint(__ldg(reinterpret_cast<const float*>(rays + st.slot) + 7));
+            const uint32_t kind = (fl >> 16) & 3u, bit = (fl >> 8) & 0xFFu;
             atomicOr(out_words + 8u * p + 4u + kind, 1u << bit);
         }
     }
     __device__ __forceinline__ void skip(uint32_t) const {}
+    __device__ __forceinline__ bool wants_nid() const { return false; }
+    __device__ __forceinline__ bool wants_bary() const { return false; }
 };
 
 // -------------------------------------------------------------------- persistent loop
 
+// The work items of a launch: the policy's own count, or the launch's.
+template <class P, class = void>
+struct counts_items { static constexpr bool value = false; };
+template <class P>
+struct counts_items<P, decltype((void)&P::items)> { static constexpr bool value = true; };
+template <class Policy>
+__device__ __forceinline__ uint32_t items_of(const Policy& P, uint32_t n) {
+    if constexpr (counts_items<Policy>::value) return P.items();
+    else return n;
+}
+
+// Hands the items of a batch that a filtering policy (filters<Policy>) keeps to the
+// idle lanes of a warp: 32 items at a time are looked at, those kept wait in `pool`
+// (32 words of shared memory a warp) until lanes take them. start(item) is called by
+// the lanes that got one; sets exhausted once the batch is used up.
+template <class Policy, class Start>
+__device__ __forceinline__ void refill_filtered(const Policy& P, uint32_t n, uint32_t* counter, uint32_t* pool,
+                                                uint32_t need, uint32_t& used, uint32_t& have, bool& exhausted,
+                                                Start start) {
+    const uint32_t lane = threadIdx.x & 31u;
+    while (need) {
+        if (used == have) {
+            uint32_t base = 0;
+            if (lane == 0u) base = atomicAdd(counter, 32u);
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            if (base >= n) {
+                exhausted = true;
+                return;
+            }
+            const uint32_t item = base + lane;
+            const bool mine = item < n && P.keeps(item);
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine);
+            if (mine) pool[__popc(m & lanemask_lt())] = item;
+            __syncwarp();
+            used = 0;
+            have = (uint32_t)__popc(m);
+            continue;
+        }
+        const uint32_t r = (uint32_t)__popc(need & lanemask_lt());
+        const bool take = ((need >> lane) & 1u) && r < have - used;
+        if (take) start(pool[used + r]);
+        __syncwarp();
+        used = min(have, used + (uint32_t)__popc(need));
+        need &= ~__ballot_sync(0xFFFFFFFFu, take);
+    }
+}
+
 // sdepth: traversal-stack entries per thread (the tree depth; <= 32). The stack
-// lives in dynamic shared memory, entry k of thread t at [k * BLOCK + t]
-// (binary form) or [(2k, 2k+1) * BLOCK + t] (8-wide form).
+// lives in dynamic shared memory, entry k of thread t at [k * BLOCK + t].
 template <int BLOCK, bool WIDE, bool STATS, class Policy>
 __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_persistent(SceneView s, Policy P, uint32_t n_static,
-                                                      const uint32_t* n_dev, uint32_t* counter, uint32_t* err,
+                                                      uint32_t* counter, uint32_t* err,
                                                       unsigned long long* stats, int sdepth, int knobs) {
     extern __shared__ uint32_t stack_mem[];
     // knobs: refill threshold (bits 0..7), phase-switch threshold (bits 8..15)
@@ -254,8 +344,10 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
     const uint32_t phase_sw = (uint32_t)(knobs >> 8) & 0xFFu;
     uint32_t* stk = stack_mem + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = n_dev ? *n_dev : n_static;
+    const uint32_t n = items_of(P, n_static);
     const uint32_t root = s.num_nodes == 1u ? kNidLeafBit : 0u;   // baseRaytracingPass.glsl:20
+    uint32_t* pool = stack_mem + (size_t)sdepth * BLOCK + (threadIdx.x & ~31u);   // filters<Policy> only
+    uint32_t used = 0, have = 0;
 
     TravState st;
     st.done = true;
@@ -265,6 +357,18 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
     // converged instead of once per lane as lanes end at different steps.
     bool active = false, pending = false, exhausted = false;
     uint32_t idx = 0;
+    auto start = [&](uint32_t item) {
+        idx = item;
+        if (P.load(s, idx, st)) {
+            st.t0 = st.t;
+            st.err = err;
+            if (WIDE) wide_init(s, st, stk);
+            else trav_init(st, root);
+            active = true;
+        } else {
+            P.skip(idx);
+        }
+    };
     for (;;) {
         const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !active);
         // refill once at least refill_min lanes are idle (32: whole-warp
@@ -284,27 +388,20 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
                     atomicAdd(stats + 4, (unsigned long long)st.c_reload);
                 }
             }
-            if constexpr (finishes<Policy>::value) P.finished(stored, st.slot);
+            if constexpr (finishes<Policy>::value) P.finished(stored, st.slot2);
             if (!exhausted) {
-                const uint32_t need = __ballot_sync(0xFFFFFFFFu, !active);
-                const int leader = __ffs(need) - 1;
-                uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(need));
-                base = __shfl_sync(0xFFFFFFFFu, base, leader);
-                if ((uint64_t)base + (uint32_t)__popc(need) >= n) exhausted = true;
-                if (!active) {
-                    const uint32_t my = base + __popc(need & lanemask_lt());
-                    if (my < n) {
-                        idx = my;
-                        if (P.load(s, idx, st)) {
-                            st.t0 = st.t;
-                            st.err = err;
-                            if (WIDE) wide_init(s, st, stk);
-                            else trav_init(st, root);
-                            active = true;
-                        } else {
-                            P.skip(idx);
-                        }
+                const uint32_t need = idle;
+                if constexpr (filters<Policy>::value) {
+                    refill_filtered(P, n, counter, pool, need, used, have, exhausted, start);
+                } else {
+                    const int leader = __ffs(need) - 1;
+                    uint32_t base = 0;
+                    if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(need));
+                    base = __shfl_sync(0xFFFFFFFFu, base, leader);
+                    if ((uint64_t)base + (uint32_t)__popc(need) >= n) exhausted = true;
+                    if (!active) {
+                        const uint32_t my = base + __popc(need & lanemask_lt());
+                        if (my < n) start(my);
                     }
                 }
             }
@@ -323,6 +420,102 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
             pending = true;
         }
     }
+}
+
+// Rays of one kind on their own tree: any-hit rays on the 4-wide one (trace_any.cuh),
+// closest-hit rays on the binary one's child pairs (trace_pair.cuh). The same
+// persistent loop, with the ray's place in st.node alone -- an inner node, a leaf, or
+// kAnyIdle, which is also the lowest word of its stack, so that popping it ends the
+// walk. sdepth: stack words per thread; an any-hit ray that would need more takes the
+// plain binary walk, a closest-hit ray never does.
+//
+// A batch of both kinds is two launches (kPairFirst, kPairSecond) that may overlap: the
+// first lets the second start as soon as its own blocks leave room, so that the second's
+// rays fill the first's tail; neither reads what the other writes, and the second ends
+// only after the first has.
+constexpr int kAlone = 0, kPairFirst = 1, kPairSecond = 2;
+template <int BLOCK, bool ANY, class Policy>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_walk(SceneView s, Policy P, uint32_t n_static, uint32_t* counter,
+                                                              uint32_t* err, int sdepth, int knobs) {
+    extern __shared__ uint32_t stack_mem[];
+    // knobs: refill threshold (bits 0..7), phase-switch threshold (bits 8..15), role in a pair (bits 16..)
+    if ((knobs >> 16) == kPairFirst) cudaTriggerProgrammaticLaunchCompletion();
+    const int refill_min = knobs & 0xFF;
+    const uint32_t phase_sw = (uint32_t)(knobs >> 8) & 0xFFu;
+    uint32_t* stk = stack_mem + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = items_of(P, n_static);
+    uint32_t* org = stk + (size_t)sdepth * BLOCK;   // the ray's origin (any-hit) and direction
+    uint32_t* dir = org + 3 * BLOCK;
+    uint32_t* pool = stack_mem + (size_t)(sdepth + 6) * BLOCK + (threadIdx.x & ~31u);   // filters<Policy> only
+    uint32_t used = 0, have = 0;
+    const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(stk);
+    const uint32_t limit = bottom + ((uint32_t)sdepth - 5u) * BLOCK * 4u;   // an any-hit visit pushes up to four words
+
+    TravState st;
+    st.node = kAnyIdle;
+    bool pending = false, exhausted = false;
+    uint32_t idx = 0;
+    stk[0] = kAnyIdle;
+    auto start = [&](uint32_t item) {
+        idx = item;
+        if (P.load(s, idx, st)) {
+            if (ANY) any_init(s, st, bottom);
+            else pair_init(s, st, bottom);
+            if (ANY) put3<BLOCK>(org, st.r.ox, st.r.oy, st.r.oz);
+            put3<BLOCK>(dir, st.r.dx, st.r.dy, st.r.dz);
+            pending = true;
+        } else {
+            P.skip(idx);
+        }
+    };
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, st.node == kAnyIdle);
+        if (idle && (exhausted || __popc(idle) >= refill_min || idle == 0xFFFFFFFFu)) {
+            const bool stored = pending && st.node == kAnyIdle;
+            if (stored) {
+                pending = false;
+                st.any = ANY;
+                if (ANY) get3<BLOCK>(org, st.r.ox, st.r.oy, st.r.oz);
+                get3<BLOCK>(dir, st.r.dx, st.r.dy, st.r.dz);
+                if (ANY) any_finish_or_walk(s, st, err);
+                else pair_finish(s, st, P.wants_nid(), P.wants_bary());
+                P.store(s, idx, st, st.t);   // an any-hit ray's t stays its tmax
+            }
+            if constexpr (finishes<Policy>::value) P.finished(stored, st.slot2);
+            if (exhausted) {
+                if (idle == 0xFFFFFFFFu) break;
+            } else if constexpr (filters<Policy>::value) {
+                refill_filtered(P, n, counter, pool, idle, used, have, exhausted, start);
+            } else {
+                const int leader = __ffs(idle) - 1;
+                uint32_t base = 0;
+                if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(idle));
+                base = __shfl_sync(0xFFFFFFFFu, base, leader);
+                if ((uint64_t)base + (uint32_t)__popc(idle) >= n) exhausted = true;
+                const uint32_t my = base + __popc(idle & lanemask_lt());
+                if (((idle >> lane) & 1u) && my < n) start(my);
+            }
+        }
+        for (;;) {   // node rounds (see plain_step_warp)
+            const uint32_t nm = __ballot_sync(0xFFFFFFFFu, (int)st.node >= 0);
+            if (nm == 0u) break;
+            if ((uint32_t)__popc(nm) <= phase_sw &&
+                __any_sync(0xFFFFFFFFu, (int)st.node < 0 && st.node != kAnyIdle)) break;
+            if ((int)st.node >= 0) {
+                if (ANY) any_advance<BLOCK>(s, st, limit);
+                else pair_advance<BLOCK>(s, st, dir);
+            }
+        }
+        if ((int)st.node < 0 && st.node != kAnyIdle) {
+            Ray r{st.r.ox, st.r.oy, st.r.oz, 0.f, 0.f, 0.f};
+            if (ANY) get3<BLOCK>(org, r.ox, r.oy, r.oz);
+            get3<BLOCK>(dir, r.dx, r.dy, r.dz);
+            if (ANY) any_leaf<BLOCK>(s, st, r);
+            else pair_leaf<BLOCK>(s, st, r);
+        }
+    }
+    if ((knobs >> 16) == kPairSecond) cudaGridDependencySynchronize();
 }
 
 // -------------------------------------------------------------------- secondary ray generation
@@ -538,23 +731,28 @@ __global__ void __launch_bounds__(256) k_gen_secondary(SceneView s, GenParams g)
     }
 }
 
-// prefix[b * kNumKinds + k] = first work item of band b's kind k over the
-// (capacity-clamped) segment counts. A band without secondary rays is final
-// already: its flag (when there are flags) is raised here.
-__global__ void k_kind_prefix(const uint32_t* q_counts, uint32_t* prefix, QueueBands qb, volatile uint32_t* flags) {
+// prefix[e] = first work item of segment e (see SecondaryPolicy) over the
+// (capacity-clamped) segment counts, and the rays per band. A band without secondary
+// rays is final already: its flag (when there are flags) is raised here.
+__global__ void k_kind_prefix(const uint32_t* q_counts, uint32_t* prefix, uint32_t* band_total, QueueBands qb,
+                              bool closest_last, volatile uint32_t* flags) {
     uint32_t acc = 0;
+    for (uint32_t e = 0; e < qb.n * kNumKinds; ++e) {
+        uint32_t band, kind;
+        segment_of(e, qb.n, closest_last, band, kind);
+        prefix[e] = acc;
+        acc += min(q_counts[band * kNumKinds + kind], qb.cap[band]);
+    }
+    prefix[qb.n * kNumKinds] = acc;
     for (uint32_t b = 0; b < qb.n; ++b) {
-        const uint32_t first = acc;
-        for (uint32_t k = 0; k < kNumKinds; ++k) {
-            prefix[b * kNumKinds + k] = acc;
-            acc += min(q_counts[b * kNumKinds + k], qb.cap[b]);
-        }
-        if (flags && acc == first) {
+        uint32_t t = 0;
+        for (uint32_t k = 0; k < kNumKinds; ++k) t += min(q_counts[b * kNumKinds + k], qb.cap[b]);
+        band_total[b] = t;
+        if (flags && t == 0u) {
             __threadfence_system();
             flags[b] = 1u;
         }
     }
-    prefix[qb.n * kNumKinds] = acc;
 }
 
 // Adds the frame's ray count (primary rays of rows 1..H-1 plus the secondary queue).
@@ -633,55 +831,108 @@ __global__ void __launch_bounds__(256) k_cull_lights(SceneView s, tim_rt_pass_da
 
 // -------------------------------------------------------------------- launchers
 
-template <int BLOCK, bool WIDE>
+// One word per stack entry, and a filtering policy's 32 words a warp of items not yet handed out.
+template <int BLOCK, class Policy>
 constexpr size_t stack_bytes(int depth) {
-    return sizeof(uint32_t) * (size_t)depth * BLOCK;   // one word per entry in both forms
+    return sizeof(uint32_t) * (size_t)(depth + (filters<Policy>::value ? 1 : 0)) * BLOCK;
 }
 
-// Grid of the persistent kernels: as many resident blocks as the occupancy
+// Grid of a persistent kernel: as many resident blocks as the occupancy
 // calculator allows on every SM for this stack depth (cached per device and depth).
-template <int BLOCK, bool WIDE, bool STATS, class Policy>
-static int grid_for(int depth) {
-    static GridCache cache;
-    return cache.get(depth, [depth](int dev) {
+template <int BLOCK, class Policy, class K>
+static int grid_of(GridCache& cache, K* kernel, int depth, int max_depth) {
+    return cache.get(depth, [=](int dev) {
         int sms = 0, per = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(k_persistent<BLOCK, WIDE, STATS, Policy>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)stack_bytes<BLOCK, WIDE>(kStackSize));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_persistent<BLOCK, WIDE, STATS, Policy>, BLOCK,
-                                                      stack_bytes<BLOCK, WIDE>(depth));
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stack_bytes<BLOCK, Policy>(max_depth));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, BLOCK, stack_bytes<BLOCK, Policy>(depth));
         return (sms > 0 ? sms : 1) * (per > 0 ? per : 1);
     });
 }
 
 template <int BLOCK, bool WIDE, bool STATS, class Policy>
-static void launch_block(const SceneView& s, const Policy& P, uint32_t n_static, const uint32_t* n_dev,
+static void launch_block(const SceneView& s, const Policy& P, uint32_t n_static,
                          uint32_t* counter, uint32_t* err, unsigned long long* stats, int depth, int refill,
                          cudaStream_t stream) {
-    k_persistent<BLOCK, WIDE, STATS, Policy><<<grid_for<BLOCK, WIDE, STATS, Policy>(depth), BLOCK,
-                                               stack_bytes<BLOCK, WIDE>(depth), stream>>>(s, P, n_static, n_dev,
-                                                                                          counter, err, stats, depth,
-                                                                                          refill);
+    static GridCache cache;
+    const int grid = grid_of<BLOCK, Policy>(cache, k_persistent<BLOCK, WIDE, STATS, Policy>, depth, kStackSize);
+    k_persistent<BLOCK, WIDE, STATS, Policy><<<grid, BLOCK, stack_bytes<BLOCK, Policy>(depth), stream>>>(
+        s, P, n_static, counter, err, stats, depth, refill);
 }
 
 template <bool WIDE, class Policy>
-static cudaError_t launch_persistent(const SceneView& s, const Policy& P, uint32_t n_static, const uint32_t* n_dev,
+static cudaError_t launch_persistent(const SceneView& s, const Policy& P, uint32_t n_static,
                                      uint32_t* counter, uint32_t* err, cudaStream_t stream, const LaunchConfig& cfg) {
     int depth = WIDE ? (int)s.wide_depth : (int)s.depth;
     if (cfg.stack_depth > depth) depth = cfg.stack_depth;
     depth = depth < 1 ? 1 : (depth > kStackSize ? kStackSize : depth);
     const int refill = launch_knobs(cfg);
     if (cfg.stats) {
-        launch_block<128, WIDE, true>(s, P, n_static, n_dev, counter, err, cfg.stats, depth, refill, stream);
+        launch_block<128, WIDE, true>(s, P, n_static, counter, err, cfg.stats, depth, refill, stream);
         return cudaGetLastError();
     }
     switch (cfg.block) {
-        case 64: launch_block<64, WIDE, false>(s, P, n_static, n_dev, counter, err, nullptr, depth, refill, stream); break;
-        case 256: launch_block<256, WIDE, false>(s, P, n_static, n_dev, counter, err, nullptr, depth, refill, stream); break;
-        default: launch_block<128, WIDE, false>(s, P, n_static, n_dev, counter, err, nullptr, depth, refill, stream); break;
+        case 64: launch_block<64, WIDE, false>(s, P, n_static, counter, err, nullptr, depth, refill, stream); break;
+        case 256: launch_block<256, WIDE, false>(s, P, n_static, counter, err, nullptr, depth, refill, stream); break;
+        default: launch_block<128, WIDE, false>(s, P, n_static, counter, err, nullptr, depth, refill, stream); break;
     }
     return cudaGetLastError();
 }
+
+// Most stack words of an any-hit and a closest-hit ray of k_walk. 24 against 16 words:
+// the frame's any-hit rays the same, those of a probe update in 1M triangles 1.60
+// against 2.01 ms (16 overflow often enough there for the binary walk to show).
+constexpr int kAnyStack = 24, kWalkStack = kStackSize + 2;
+
+template <int BLOCK, bool ANY, class Policy>
+static cudaError_t launch_walk_block(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter,
+                                     uint32_t* err, int depth, int knobs, int role, int share, cudaStream_t stream) {
+    static GridCache cache;
+    const int words = depth + 6;   // and the ray's origin and direction
+    const int grid = grid_of<BLOCK, Policy>(cache, k_walk<BLOCK, ANY, Policy>, words, kWalkStack + 6);
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(share > 1 && grid >= share ? grid / share : grid);
+    lc.blockDim = dim3(BLOCK);
+    lc.dynamicSmemBytes = stack_bytes<BLOCK, Policy>(words);
+    lc.stream = stream;
+    cudaLaunchAttribute at{};
+    if (role == kPairSecond) {
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&lc, k_walk<BLOCK, ANY, Policy>, s, P, n_static, counter, err, depth, knobs | role << 16);
+}
+
+// One launch of k_walk, or one of a pair (of which the first may be given a share of the
+// GPU only). Stack words: a closest-hit ray leaves one child a level waiting, an any-hit
+// ray up to three slots, of which kAnyStack words are kept; the end marker; and the word
+// above the top, which a push writes whether it keeps it or not.
+template <bool ANY, class Policy>
+static cudaError_t launch_walk(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter, uint32_t* err,
+                               cudaStream_t stream, const LaunchConfig& cfg, int role = kAlone, int share = 1) {
+    int depth = (int)s.depth + 2;
+    LaunchConfig c = cfg;
+    if (ANY) {
+        depth = 3 * (int)s.depth4 + 2;
+        depth = depth < 6 ? 6 : (depth > kAnyStack ? kAnyStack : depth);
+        // any-hit rays of one origin's neighbourhood profit more from starting together (they
+        // read the same nodes; the L1 binds this walk): 16 -> 24 idle lanes, 0.81 -> 0.73 ms
+        // for the 5.1M any-hit rays of the 1080p frame. launch_knobs limits it to 32.
+        c.refill_min = cfg.refill_min + cfg.refill_min / 2;
+    }
+    const int knobs = launch_knobs(c);
+    switch (cfg.block) {
+        case 64: return launch_walk_block<64, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
+        case 256: return launch_walk_block<256, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
+        default: return launch_walk_block<128, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
+    }
+}
+
+// Launches of the binary form take the two trees where the scene has them; the
+// counting kernels count the plain binary walk's work.
+static bool use_four(const SceneView& s, const LaunchConfig& cfg) { return !cfg.wide && s.nodes4 && !cfg.stats; }
 
 cudaError_t launch_trace_batch(const SceneView& s, const tim_rt_ray* rays, uint32_t n, uint32_t mode, uint32_t* hit,
                                uint32_t* nid, float* bary, uint32_t* counter, uint32_t* err, cudaStream_t stream,
@@ -690,10 +941,53 @@ cudaError_t launch_trace_batch(const SceneView& s, const tim_rt_ray* rays, uint3
     if (mode & TIM_RT_TRACE_TLAS) {   // any-hit only, binary form only (checked by the callers)
         TlasBatchPolicy T;
         static_cast<BatchPolicy&>(T) = P;
-        return launch_persistent<false>(s, T, n, nullptr, counter, err, stream, cfg);
+        return launch_persistent<false>(s, T, n, counter, err, stream, cfg);
     }
-    if (cfg.wide) return launch_persistent<true>(s, P, n, nullptr, counter, err, stream, cfg);
-    return launch_persistent<false>(s, P, n, nullptr, counter, err, stream, cfg);
+    if (cfg.wide) return launch_persistent<true>(s, P, n, counter, err, stream, cfg);
+    if (!use_four(s, cfg)) return launch_persistent<false>(s, P, n, counter, err, stream, cfg);
+    if (P.mode == TIM_RT_MODE_CLOSEST) return launch_walk<false>(s, P, n, counter, err, stream, cfg);
+    if (P.mode == TIM_RT_MODE_ANY) return launch_walk<true>(s, P, n, counter, err, stream, cfg);
+    KindBatchPolicy K;
+    static_cast<BatchPolicy&>(K) = P;
+    K.kind = 0u;
+    const cudaError_t e = launch_walk<false>(s, K, n, counter, err, stream, cfg, kPairFirst);
+    if (e != cudaSuccess) return e;
+    K.kind = TIM_RT_RAY_ANY;
+    return launch_walk<true>(s, K, n, counter + 1, err, stream, cfg, kPairSecond);
+}
+
+// Traces the secondary queue (counts in q_counts, laid out as kernels.h says): the
+// segments' first items, then the rays -- in one launch, or, with the 4-wide tree, the
+// any-hit rays and the bounce rays in launches of their own, since they walk different
+// trees and a warp of both kinds would walk each with part of its lanes.
+static cudaError_t launch_secondary(const SceneView& s, SecondaryPolicy P, uint32_t* counters, uint32_t* err,
+                                    cudaStream_t stream, const LaunchConfig& cfg, bool bounces, cudaEvent_t start) {
+    const uint32_t nb = P.qb.n;
+    uint32_t* prefix = counters + 2u + kNumKinds * nb;
+    uint32_t* band_total = prefix + kNumKinds * nb + 1u + nb;
+    const bool four = use_four(s, cfg);
+    P.prefix = prefix;
+    P.band_total = band_total;
+    P.done = P.flags ? prefix + kNumKinds * nb + 1u : nullptr;
+    P.closest_last = four;
+    P.seg0 = 0u;
+    P.seg1 = nb * kNumKinds;
+    k_kind_prefix<<<1, 1, 0, stream>>>(counters + 2, prefix, band_total, P.qb, four, P.flags);
+    if (start) cudaEventRecord(start, stream);
+    if (cfg.wide) return launch_persistent<true>(s, P, 0u, counters + 1, err, stream, cfg);
+    if (!four) return launch_persistent<false>(s, P, 0u, counters + 1, err, stream, cfg);
+    if (bounces) {
+        P.seg0 = nb * kKindBounce;
+        // with bands both launches must get on together, as a band is final after both:
+        // half of the GPU for the bounce rays (the 1080p frame through host buffers takes
+        // 2.57 ms with a half, 2.58 with a third, 2.62 with a quarter)
+        const cudaError_t e = launch_walk<false>(s, P, 0u, counters + 3u + 54u * nb, err, stream, cfg, kPairFirst,
+                                                 nb > 1u ? 2 : 1);
+        if (e != cudaSuccess) return e;
+        P.seg0 = 0u;
+    }
+    P.seg1 = nb * kKindBounce;
+    return launch_walk<true>(s, P, 0u, counters + 1, err, stream, cfg, bounces ? kPairSecond : kAlone);
 }
 
 uint32_t camera_queue_segment(uint32_t W, uint32_t H) { return W * H; }
@@ -736,8 +1030,6 @@ cudaError_t launch_camera(const SceneView& s, const tim_rt_pass_data& pd, uint32
     // counters: [0] pixel work, [1] secondary work, then the bands' kind counts, their
     // prefix and the bands' finished rays
     uint32_t* q_counts = counters + 2;
-    uint32_t* prefix = counters + 2 + kNumKinds * qb.n;
-    uint32_t* done = prefix + kNumKinds * qb.n + 1u;
     CameraPolicy CP{pd, ngy16, reinterpret_cast<uint4*>(out), leaf_nid, item0};
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[0], stream);
     // primary rays: a warp refills only when all 32 lanes are idle, so it always
@@ -746,8 +1038,9 @@ cudaError_t launch_camera(const SceneView& s, const tim_rt_pass_data& pd, uint32
     LaunchConfig pcfg = cfg;
     pcfg.refill_min = 32;
     if (flags & TIM_RT_CAM_PRIMARY_BINARY) pcfg.wide = false;
-    cudaError_t e = pcfg.wide ? launch_persistent<true>(s, CP, items, nullptr, counters + 0, err, stream, pcfg)
-                              : launch_persistent<false>(s, CP, items, nullptr, counters + 0, err, stream, pcfg);
+    cudaError_t e = pcfg.wide ? launch_persistent<true>(s, CP, items, counters + 0, err, stream, pcfg)
+                    : use_four(s, pcfg) ? launch_walk<false>(s, CP, items, counters + 0, err, stream, pcfg)
+                                        : launch_persistent<false>(s, CP, items, counters + 0, err, stream, pcfg);
     if (e != cudaSuccess) return e;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[1], stream);
     GenParams g;
@@ -769,15 +1062,18 @@ cudaError_t launch_camera(const SceneView& s, const tim_rt_pass_data& pd, uint32
     g.item1 = item1;
     k_gen_secondary<<<(items + 255u) / 256u, 256, 0, stream>>>(s, g);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_kind_prefix<<<1, 1, 0, stream>>>(q_counts, prefix, qb, flags_host);
-    if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[2], stream);
-    SecondaryPolicy SP{q_rays, q_pixel, prefix, qb, out, reinterpret_cast<uint4*>(bounce_out),
-                       flags_host ? done : nullptr, flags_host};
+    SecondaryPolicy SP{};
+    SP.rays = q_rays;
+    SP.pixel = q_pixel;
+    SP.qb = qb;
+    SP.out_words = out;
+    SP.bounce_out = reinterpret_cast<uint4*>(bounce_out);
+    SP.flags = flags_host;
     LaunchConfig cfg2 = cfg;   // the secondary kernel counts into stats[8..12]
     if (cfg.stats) cfg2.stats = cfg.stats + 8;
-    const uint32_t* total = prefix + kNumKinds * qb.n;
-    e = cfg.wide ? launch_persistent<true>(s, SP, 0u, total, counters + 1, err, stream, cfg2)
-                 : launch_persistent<false>(s, SP, 0u, total, counters + 1, err, stream, cfg2);
+    e = launch_secondary(s, SP, counters, err, stream, cfg2, (flags & TIM_RT_CAM_BOUNCE) != 0u,
+                         cfg.phase_ev ? cfg.phase_ev[2] : nullptr);
+    const uint32_t* total = counters + 2u + 2u * kNumKinds * qb.n;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[3], stream);
     if (e != cudaSuccess || !d_ray_count) return e;
     // primary rays of the rows traced (output row 0 is never traced)
@@ -868,6 +1164,8 @@ struct ProbePolicy {
         leaf_nid[st.slot] = st.hit ? st.nid : 0xFFFFFFFFu;
     }
     __device__ __forceinline__ void skip(uint32_t) const {}
+    __device__ __forceinline__ bool wants_nid() const { return true; }
+    __device__ __forceinline__ bool wants_bary() const { return false; }
 };
 
 // Shadow rays of the probe hits: the sun (tmax = TMAX) and the hit leaf's lights
@@ -1293,12 +1591,13 @@ cudaError_t launch_probes(const SceneView& s, const ProbeArgs& d, uint32_t* out,
                           float* octa, uint32_t side, cudaStream_t stream, const LaunchConfig& cfg) {
     const uint32_t n = d.np * d.nd;
     uint32_t* q_counts = counters + 2;
-    uint32_t* prefix = counters + 2 + kNumKinds;
     ProbePolicy PP{d, reinterpret_cast<uint4*>(out), leaf_nid};
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[0], stream);
-    const bool probe_wide = cfg.wide && !cfg.primary_binary;
-    cudaError_t e = probe_wide ? launch_persistent<true>(s, PP, n, nullptr, counters + 0, err, stream, cfg)
-                               : launch_persistent<false>(s, PP, n, nullptr, counters + 0, err, stream, cfg);
+    LaunchConfig pcfg = cfg;
+    pcfg.wide = cfg.wide && !cfg.primary_binary;
+    cudaError_t e = pcfg.wide ? launch_persistent<true>(s, PP, n, counters + 0, err, stream, pcfg)
+                    : use_four(s, pcfg) ? launch_walk<false>(s, PP, n, counters + 0, err, stream, pcfg)
+                                        : launch_persistent<false>(s, PP, n, counters + 0, err, stream, pcfg);
     if (e != cudaSuccess) return e;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[1], stream);
     GenParams g{};
@@ -1310,13 +1609,14 @@ cudaError_t launch_probes(const SceneView& s, const ProbeArgs& d, uint32_t* out,
     g.qb.cap[0] = n;
     k_probe_gen<<<(n + 255u) / 256u, 256, 0, stream>>>(s, d, g, leaf_nid);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_kind_prefix<<<1, 1, 0, stream>>>(q_counts, prefix, g.qb, nullptr);
-    if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[2], stream);
-    SecondaryPolicy SP{q_rays, q_pixel, prefix, g.qb, out, nullptr, nullptr, nullptr};
+    SecondaryPolicy SP{};
+    SP.rays = q_rays;
+    SP.pixel = q_pixel;
+    SP.qb = g.qb;
+    SP.out_words = out;
     LaunchConfig cfg2 = cfg;
     if (cfg.stats) cfg2.stats = cfg.stats + 8;
-    e = cfg.wide ? launch_persistent<true>(s, SP, 0u, prefix + kNumKinds, counters + 1, err, stream, cfg2)
-                 : launch_persistent<false>(s, SP, 0u, prefix + kNumKinds, counters + 1, err, stream, cfg2);
+    e = launch_secondary(s, SP, counters, err, stream, cfg2, false, cfg.phase_ev ? cfg.phase_ev[2] : nullptr);
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[3], stream);
     if (e != cudaSuccess) return e;
     k_probe_light<<<(n + 255u) / 256u, 256, 0, stream>>>(s, d, out, irr);

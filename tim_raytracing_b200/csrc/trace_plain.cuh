@@ -42,6 +42,11 @@ struct TravState {
     bool near2;         // closest: another hit t2 has RN(t2 - 1e-5) <= t1
     bool dup_ok;        // closest: the hit leaf's id is not an output (see wide_leaf)
     uint32_t leaf;      // pending leaf slot of the current wide node (8 = none)
+    // any-hit rays on the 4-wide tree (trace_any.cuh): the addends of the near and far
+    // planes per axis
+    float anx, any_, anz, afx, afy, afz;
+    const char *px, *py, *pz;   // where the ray reads an axis' planes, for node 0
+    uint32_t top;               // shared-memory address of the stack's top word
     uint32_t* err;      // two-level walk: the device error word (a nested walk's stack guard)
 };
 
