@@ -262,7 +262,7 @@ int tim_rt_destroy(tim_rt_ctx* c) {
     c->batches.clear();
     for (auto& kv : c->scenes) {
         Scene* s = kv.second.get();
-        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
+        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->trees}) dev_free(c, *b);
     }
     c->scenes.clear();
     for (DevBuf* b : {&c->rays, &c->hits, &c->nid, &c->bary, &c->counters, &c->cam_out, &c->cam_bounce, &c->cam_nid,
@@ -335,7 +335,8 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
     const uint8_t* blob = static_cast<const uint8_t*>(bvh_bytes);
     std::string err;
     uint32_t depth = 0;
-    if (!validate_bvh(blob, n_bytes, ranges, pc->numNodes, num_vertex, pc->numLights, pc->numBlas, &depth, err)) {
+    uint64_t tris = 0;
+    if (!validate_bvh(blob, n_bytes, ranges, pc->numNodes, num_vertex, pc->numLights, pc->numBlas, &depth, err, &tris)) {
         set_error("tim_rt_upload_bvh: " + err);
         return TIM_RT_EINVAL;
     }
@@ -373,27 +374,16 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
             return TIM_RT_EUNSUPPORTED;
         }
     }
-    // the plain form's leaf-triangle copy (16-byte vector fetches instead of
-    // scalar gathers of the records and vertex positions)
-    RawVec<float> ptris;
-    RawVec<uint32_t> pleaf;
-    build_leaf_tris(blob, ranges, pc->numNodes, pos, ptris, pleaf);
     auto fail = [&](int code) {
-        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
+        for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->trees}) dev_free(c, *b);
         return code;
     };
     if ((rc = dev_alloc(c, s->blob, n_bytes))) return fail(rc);
     if ((rc = dev_alloc(c, s->pos, 12ull * max_vertex))) return fail(rc);
     if (nrm && (rc = dev_alloc(c, s->nrm, 12ull * max_vertex))) return fail(rc);
     if (uv && (rc = dev_alloc(c, s->uv, 8ull * max_vertex))) return fail(rc);
-    if ((rc = dev_alloc(c, s->pleaf, 4ull * pleaf.size()))) return fail(rc);
-    if (!ptris.empty() && (rc = dev_alloc(c, s->ptris, 4ull * ptris.size()))) return fail(rc);
-    if (cudaMemcpyAsync(s->pleaf.ptr, pleaf.data(), 4ull * pleaf.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-        (!ptris.empty() &&
-         cudaMemcpyAsync(s->ptris.ptr, ptris.data(), 4ull * ptris.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess)) {
-        set_error("tim_rt_upload_bvh: host-to-device copy of the leaf triangles failed");
-        return fail(TIM_RT_EDEVICE);
-    }
+    if ((rc = dev_alloc(c, s->pleaf, 16ull * pc->numNodes))) return fail(rc);
+    if (tris && (rc = dev_alloc(c, s->ptris, 48ull * tris))) return fail(rc);
     if (cudaMemcpyAsync(s->blob.ptr, blob, n_bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
         cudaMemcpyAsync(s->pos.ptr, pos, 12ull * num_vertex, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
         (nrm && cudaMemcpyAsync(s->nrm.ptr, nrm, 12ull * num_vertex, cudaMemcpyHostToDevice, c->stream) != cudaSuccess) ||
@@ -412,10 +402,6 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
             return fail(TIM_RT_EDEVICE);
         }
         s->has_wide = true;
-    }
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
-        set_error("tim_rt_upload_bvh: stream synchronisation failed");
-        return fail(TIM_RT_EDEVICE);
     }
     const uint8_t* d = static_cast<const uint8_t*>(s->blob.ptr);
     SceneView& v = s->view;
@@ -439,12 +425,20 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
     v.wide_root_is_leaf = wh.root_is_leaf;
     v.pleaf = static_cast<const uint4*>(s->pleaf.ptr);
     v.ptris = static_cast<const float4*>(s->ptris.ptr);
+    if (build_leaf_tris(s.get(), c->stream) != cudaSuccess) {
+        set_error("tim_rt_upload_bvh: building the leaf triangles failed");
+        return fail(TIM_RT_EDEVICE);
+    }
     uint32_t root_left;   // the root's first child
     std::memcpy(&root_left, blob + ranges[TIM_RT_RANGE_NODE][0] + 8, 4);
     root_left &= 0x3FFFFFFFu;
-    if ((rc = build_four(c, s.get(), (uint32_t)(ptris.size() / 12u), root_left))) return fail(rc);
+    if ((rc = build_four(c, s.get(), tris, root_left))) return fail(rc);
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
+        set_error("tim_rt_upload_bvh: stream synchronisation failed");
+        return fail(TIM_RT_EDEVICE);
+    }
     s->bytes = s->blob.bytes + s->pos.bytes + s->nrm.bytes + s->uv.bytes + s->wnodes.bytes + s->wtris.bytes + s->wnid.bytes +
-               s->pleaf.bytes + s->ptris.bytes + s->nodes4.bytes + s->leaf4.bytes + s->tri_leaf4.bytes + s->pairs.bytes;
+               s->pleaf.bytes + s->ptris.bytes + s->trees.bytes;
     const uint32_t id = c->next_id++;
     c->scenes[id] = std::move(s);
     *out = id;
@@ -477,7 +471,7 @@ int tim_rt_free_scene(tim_rt_ctx* c, tim_rt_scene_id id) {
         return TIM_RT_EINVAL;
     }
     cudaStreamSynchronize(c->stream);
-    for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
+    for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->trees}) dev_free(c, *b);
     c->scenes.erase(id);
     return TIM_RT_OK;
 }

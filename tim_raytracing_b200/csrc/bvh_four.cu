@@ -1,6 +1,6 @@
 // bvh_four.cu -- the trees the binary form's rays walk, built on the GPU from an uploaded
-// scene's binary tree: the 4-wide tree of the any-hit rays (trace_any.cuh) and the
-// child-pair records of the closest-hit rays (trace_pair.cuh).
+// scene's binary tree: the leaf triangles by node, the 4-wide tree of the any-hit rays
+// (trace_any.cuh) and the child-pair records of the closest-hit rays (trace_pair.cuh).
 //
 // Every 4-wide slot is one binary subtree, so a leaf of the 4-wide tree is a leaf of
 // the reference's with its triangles in their order. Which subtrees become a node's
@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
+#include <string>
 #include "common.cuh"
 #include "context.h"
 #include "kernels.h"
@@ -327,22 +328,90 @@ __global__ void k_pairs(In in, float4* pairs) {
     o[6] = make_float4(__uint_as_float(ref[0]), __uint_as_float(ref[1]), 0.f, 0.f);
 }
 
+// Per node (first triangle, leaf header, leaf-data offset, 0); a node without leaf data
+// (offset 0xFFFFFFFF) gets header 0, as the kernels read it. Per leaf-data triangle
+// record, in its leaf's order: (p0, vertexOffset) (p1 - p0, index01) (p2 - p0,
+// index2_matId), the edges being the same rounded differences CollideTriangle forms
+// (collision.glsl:60-61). A block takes the places of its nodes' triangles together
+// (blocks in any order: nothing depends on it). Runs after validate_bvh, so every offset
+// and vertex index is in range. The host loop this replaces and the copy of its result
+// were half of a 1M-triangle scene's upload.
+__global__ void __launch_bounds__(256) k_leaf_tris(SceneView s, uint32_t n, uint4* info, float4* tris) {
+    __shared__ uint32_t warp_sum[8], block_base;
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t off = 0xFFFFFFFFu, hdr = 0u;
+    if (i < n) {
+        off = reinterpret_cast<const uint4*>(s.nodes + 4u * i)->w;
+        hdr = off == 0xFFFFFFFFu ? 0u : s.leaf[off];
+    }
+    const uint32_t nt = hdr & ((1u << kTriBits) - 1u);
+    uint32_t sum = nt;
+    for (uint32_t k = 1; k < 32u; k <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, sum, k);
+        if (lane >= k) sum += v;
+    }
+    if (lane == 31u) warp_sum[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0u) {
+        uint32_t t = 0;
+        for (uint32_t k = 0; k < 8u; ++k) {
+            const uint32_t v = warp_sum[k];
+            warp_sum[k] = t;
+            t += v;
+        }
+        block_base = t ? atomicAdd(&info[0].w, t) : 0u;
+    }
+    __syncthreads();
+    if (i >= n) return;
+    const uint32_t first = block_base + warp_sum[warp] + sum - nt;
+    info[i].x = first;
+    info[i].y = hdr;
+    info[i].z = off;
+    if (i) info[i].w = 0u;
+    for (uint32_t t = 0; t < nt; ++t) {
+        const uint32_t* r = s.leaf + 1u + off + 3u * t;
+        const uint32_t r0 = r[0], r1 = r[1], r2 = r[2];
+        const float* P0 = s.pos + 3ull * (r0 + (r1 & 0xFFFFu));
+        const float* P1 = s.pos + 3ull * (r0 + (r1 >> 16));
+        const float* P2 = s.pos + 3ull * (r0 + (r2 & 0xFFFFu));
+        float4* o = tris + 3ull * (first + t);
+        o[0] = make_float4(P0[0], P0[1], P0[2], __uint_as_float(r0));
+        o[1] = make_float4(P1[0] - P0[0], P1[1] - P0[1], P1[2] - P0[2], __uint_as_float(r1));
+        o[2] = make_float4(P2[0] - P0[0], P2[1] - P0[1], P2[2] - P0[2], __uint_as_float(r2));
+    }
+}
+
 }  // namespace
 
-int build_four(tim_rt_ctx* c, Scene* s, uint32_t num_tris, uint32_t root_left) {
+cudaError_t build_leaf_tris(const Scene* s, cudaStream_t stream) {
+    const uint32_t n = s->pc.numNodes;
+    uint4* info = static_cast<uint4*>(s->pleaf.ptr);
+    cudaMemsetAsync(info, 0, 16, stream);   // node 0's unused word counts the triangles handed out
+    k_leaf_tris<<<(n + 255u) / 256u, 256, 0, stream>>>(s->view, n, info, static_cast<float4*>(s->ptris.ptr));
+    return cudaGetLastError();
+}
+
+int build_four(tim_rt_ctx* c, Scene* s, uint64_t num_tris, uint32_t root_left) {
     const uint32_t n = s->pc.numNodes;
     // With a memory budget the scene keeps to the arrays it always had, so that what
     // was admitted stays admitted; BLAS boxes are tested by the binary walk only.
-    if (c->budget || s->pc.numBlas || n < 2u || num_tris == 0u || num_tris > kFourFirstMask) return TIM_RT_OK;
+    if (c->budget || s->pc.numBlas || n < 2u || num_tris == 0u || num_tris >= kFourFirstMask) return TIM_RT_OK;
     auto up = [](uint64_t x) { return (x + 255ull) & ~255ull; };
     const uint32_t cap = n / 2u + 1u;   // inner nodes
     const uint64_t o_par = up(sizeof(Ctl)), o_arr = o_par + up(4ull * n), o_cost = o_arr + up(4ull * n),
                    o_item = o_cost + up(16ull * n), o_e = o_item + up(4ull * cap), o_base = o_e + up(sizeof(Box) * cap),
                    bytes = o_base + up(8ull * cap);
+    // No room for the trees is no error: the plain walk stays.
+    const std::string last_error = tim_rt_last_error();
+    auto alloc = [&](DevBuf& b, uint64_t size) {
+        if (dev_alloc(c, b, size) == TIM_RT_OK) return true;
+        set_error(last_error);
+        return false;
+    };
     if (c->bld.bytes < bytes) {   // the GPU builder's scratch serves here too
         cudaStreamSynchronize(c->stream);
         dev_free(c, c->bld);
-        if (dev_alloc(c, c->bld, bytes) != TIM_RT_OK) return TIM_RT_OK;   // no room for the form: the plain walk stays
+        if (!alloc(c->bld, bytes)) return TIM_RT_OK;
     }
     uint8_t* tmp = static_cast<uint8_t*>(c->bld.ptr);
     Ctl* ctl = reinterpret_cast<Ctl*>(tmp);
@@ -381,23 +450,26 @@ int build_four(tim_rt_ctx* c, Scene* s, uint32_t num_tris, uint32_t root_left) {
     const bool fits = ok && !h.bad && h.leaves && h.total < (1u << 25) && h.level[levels] == h.total && bound[0] <= 1.099511627776e12f &&
                       bound[1] <= 1.099511627776e12f && bound[2] <= 1.099511627776e12f;   // 2^40
     if (fits) {
-        if (dev_alloc(c, s->nodes4, (uint64_t)kFourBytes * h.total) == TIM_RT_OK && dev_alloc(c, s->leaf4, 32ull * h.leaves) == TIM_RT_OK &&
-            dev_alloc(c, s->tri_leaf4, 4ull * num_tris) == TIM_RT_OK && dev_alloc(c, s->pairs, (uint64_t)kPairBytes * cap) == TIM_RT_OK) {
-            k_pairs<<<blocks, 256, 0, st>>>(in, static_cast<float4*>(s->pairs.ptr));
-            k_four_fill<<<(h.total + 127u) / 128u, 128, 0, st>>>(in, cost, item, item_e, base, h.total,
-                                                                 static_cast<float4*>(s->nodes4.ptr),
-                                                                 static_cast<uint4*>(s->leaf4.ptr),
-                                                                 static_cast<uint32_t*>(s->tri_leaf4.ptr));
-            ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
-            s->view.nodes4 = static_cast<const float4*>(s->nodes4.ptr);
-            s->view.leaf4 = static_cast<const uint4*>(s->leaf4.ptr);
-            s->view.tri_leaf4 = static_cast<const uint32_t*>(s->tri_leaf4.ptr);
-            s->view.pairs = static_cast<const float4*>(s->pairs.ptr);
-            s->view.root_pair = root_left >> 1;
-            s->view.depth4 = levels;
-            for (int d = 0; d < 3; ++d) s->view.bound4[d] = bound[d];
-        } else {
-            for (DevBuf* b : {&s->nodes4, &s->leaf4, &s->tri_leaf4, &s->pairs}) dev_free(c, *b);
+        const uint64_t o_pairs = up((uint64_t)kFourBytes * h.total), o_leaf = o_pairs + up((uint64_t)kPairBytes * cap),
+                       o_tri = o_leaf + up(32ull * h.leaves);
+        if (alloc(s->trees, o_tri + 4ull * num_tris)) {
+            uint8_t* t = static_cast<uint8_t*>(s->trees.ptr);
+            SceneView& v = s->view;
+            float4* nodes4 = reinterpret_cast<float4*>(t);
+            float4* pairs = reinterpret_cast<float4*>(t + o_pairs);
+            uint4* leaf4 = reinterpret_cast<uint4*>(t + o_leaf);
+            uint32_t* tri_leaf4 = reinterpret_cast<uint32_t*>(t + o_tri);
+            k_pairs<<<blocks, 256, 0, st>>>(in, pairs);
+            k_four_fill<<<(h.total + 127u) / 128u, 128, 0, st>>>(in, cost, item, item_e, base, h.total, nodes4, leaf4,
+                                                                 tri_leaf4);
+            ok = cudaGetLastError() == cudaSuccess;
+            v.nodes4 = nodes4;
+            v.leaf4 = leaf4;
+            v.tri_leaf4 = tri_leaf4;
+            v.pairs = pairs;
+            v.root_pair = root_left >> 1;
+            v.depth4 = levels;
+            for (int d = 0; d < 3; ++d) v.bound4[d] = bound[d];
         }
     }
     if (!ok) {

@@ -22,7 +22,8 @@ bool range_ok(const uint32_t r[2], uint64_t need, uint64_t n_bytes) {
 }  // namespace
 
 bool validate_bvh(const uint8_t* blob, uint64_t n_bytes, const uint32_t ranges[7][2], uint32_t num_nodes,
-                  uint32_t num_vertex, uint32_t num_lights, uint32_t num_blas, uint32_t* depth_out, std::string& err) {
+                  uint32_t num_vertex, uint32_t num_lights, uint32_t num_blas, uint32_t* depth_out, std::string& err,
+                  uint64_t* tris_out) {
     if (!blob || num_nodes == 0) { err = "empty BVH"; return false; }
     if (ranges[TIM_RT_RANGE_NODE][0] % 16u) { err = "node range not 16-byte aligned"; return false; }
     for (int i = 0; i < 7; ++i)
@@ -36,6 +37,7 @@ bool validate_bvh(const uint8_t* blob, uint64_t n_bytes, const uint32_t ranges[7
     const uint64_t leaf_words = ranges[TIM_RT_RANGE_LEAF][1] / 4u;
     std::vector<uint8_t> depth(num_nodes, 0);
     uint32_t max_depth = 0;
+    uint64_t tris = 0;
     auto inner_ok = [&](uint32_t i) { return (nodes[i].nid[2] & kMask) != kInvalid; };
     if (num_nodes > 1 && !inner_ok(0)) { err = "root has no children"; return false; }
     for (uint32_t i = 0; i < num_nodes; ++i) {
@@ -55,6 +57,7 @@ bool validate_bvh(const uint8_t* blob, uint64_t n_bytes, const uint32_t ranges[7
             if (off >= leaf_words) { err = "node " + std::to_string(i) + ": leaf offset out of range"; return false; }
             const uint32_t hdr = leaf[off];
             const uint32_t nt = hdr & 0xFFFu, nb = (hdr >> 12) & 0xFFu, np = (hdr >> 20) & 0xFFu, nl = (hdr >> 28) & 0xFu;
+            tris += nt;
             const uint64_t end = 1ull + off + 3ull * nt + nb + np + nl;
             if (end > leaf_words) { err = "node " + std::to_string(i) + ": leaf data past the leaf range"; return false; }
             for (uint32_t t = 0; t < nt; ++t) {
@@ -73,63 +76,8 @@ bool validate_bvh(const uint8_t* blob, uint64_t n_bytes, const uint32_t ranges[7
         }
     }
     if (depth_out) *depth_out = max_depth;
+    if (tris_out) *tris_out = tris;
     return true;
-}
-
-// ---------------------------------------------------------------------------------- leaf-triangle copy
-
-// Per node: (first triangle in `tris`, leaf header word, leaf-data offset, 0); a
-// node without leaf data (offset 0xFFFFFFFF) gets header 0, as the kernels read
-// it. Per leaf-data triangle record, in node order and, within a node, in the
-// leaf's stored order: (p0, vertexOffset) (p1 - p0, index01) (p2 - p0,
-// index2_matId) as 12 floats, the edges being the same rounded differences
-// CollideTriangle forms (collision.glsl:60-61). Runs after validate_bvh, so every
-// offset and vertex index is in range.
-void build_leaf_tris(const uint8_t* blob, const uint32_t ranges[7][2], uint32_t num_nodes, const float* pos,
-                     RawVec<float>& tris, RawVec<uint32_t>& info) {
-    const PNode* nodes = reinterpret_cast<const PNode*>(blob + ranges[TIM_RT_RANGE_NODE][0]);
-    const uint32_t* leaf = reinterpret_cast<const uint32_t*>(blob + ranges[TIM_RT_RANGE_LEAF][0]);
-    info.resize(4ull * num_nodes);
-    uint64_t total = 0;
-    for (uint32_t i = 0; i < num_nodes; ++i) {
-        const uint32_t off = nodes[i].nid[3];
-        const uint32_t hdr = off == 0xFFFFFFFFu ? 0u : leaf[off];
-        info[4ull * i + 0] = (uint32_t)total;
-        info[4ull * i + 1] = hdr;
-        info[4ull * i + 2] = off;
-        info[4ull * i + 3] = 0u;
-        total += hdr & 0xFFFu;
-    }
-    tris.resize(12ull * total);
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const uint32_t chunk = (num_nodes + hw - 1u) / hw;
-    auto fill = [&](uint32_t n0, uint32_t n1) {
-        for (uint32_t i = n0; i < n1; ++i) {
-            const uint32_t nt = info[4ull * i + 1] & 0xFFFu;
-            float* out = tris.data() + 12ull * info[4ull * i];
-            for (uint32_t t = 0; t < nt; ++t, out += 12) {
-                const uint32_t* r = leaf + 1u + info[4ull * i + 2] + 3u * t;
-                const float* P0 = pos + 3ull * (r[0] + (r[1] & 0xFFFFu));
-                const float* P1 = pos + 3ull * (r[0] + (r[1] >> 16));
-                const float* P2 = pos + 3ull * (r[0] + (r[2] & 0xFFFFu));
-                for (int a = 0; a < 3; ++a) {
-                    out[a] = P0[a];
-                    out[4 + a] = P1[a] - P0[a];
-                    out[8 + a] = P2[a] - P0[a];
-                }
-                std::memcpy(out + 3, &r[0], 4);
-                std::memcpy(out + 7, &r[1], 4);
-                std::memcpy(out + 11, &r[2], 4);
-            }
-        }
-    };
-    if (total < 65536u || hw == 1u) {
-        fill(0, num_nodes);
-        return;
-    }
-    std::vector<std::thread> pool;
-    for (uint32_t n0 = 0; n0 < num_nodes; n0 += chunk) pool.emplace_back(fill, n0, std::min(num_nodes, n0 + chunk));
-    for (std::thread& t : pool) t.join();
 }
 
 // ---------------------------------------------------------------------------------- 8-wide collapse

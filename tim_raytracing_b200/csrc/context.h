@@ -20,8 +20,8 @@ struct DevBuf {
 
 struct Scene {
     DevBuf blob, pos, nrm, uv, wnodes, wtris, wnid;
-    DevBuf nodes4, leaf4, tri_leaf4, pairs;   // the any-hit and closest-hit rays' trees (build_four)
-    DevBuf ptris, pleaf;   // the plain form's leaf-triangle copy (build_leaf_tris)
+    DevBuf trees;          // the binary form's trees: nodes4, pairs, leaf4, tri_leaf4 of the view (build_four)
+    DevBuf ptris, pleaf;   // the leaf triangles by node (build_leaf_tris)
     SceneView view{};
     uint32_t ranges[7][2];
     tim_rt_push_constants pc{};
@@ -92,10 +92,13 @@ void dev_free(tim_rt_ctx* c, DevBuf& b);
 // Makes the context's device current; TIM_RT_EINVAL for a null context.
 int check_ctx(tim_rt_ctx* c);
 Scene* find_scene(tim_rt_ctx* c, tim_rt_scene_id id);
+// Fills the scene's leaf triangles (view.pleaf, view.ptris) from its uploaded nodes, leaf
+// data and positions, on the context's stream.
+cudaError_t build_leaf_tris(const Scene* s, cudaStream_t stream);
 // Builds the 4-wide tree of a scene's any-hit rays and the child-pair records of its closest-hit rays from its uploaded arrays (view
 // filled up to ptris; num_tris leaf triangles). A scene the form does not cover is
 // left without it (TIM_RT_OK, view.nodes4 null). Synchronous.
-int build_four(tim_rt_ctx* c, Scene* s, uint32_t num_tris, uint32_t root_left);
+int build_four(tim_rt_ctx* c, Scene* s, uint64_t num_tris, uint32_t root_left);
 // Stops a server's worker and releases its device memory (context teardown).
 void server_shutdown(tim_rt_ctx* c, tim_rt_server* s);
 
