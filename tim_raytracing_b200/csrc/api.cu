@@ -1019,10 +1019,8 @@ int batch_run(tim_rt_ctx* c, tim_rt_batch* b, const LaunchConfig& cfg, bool wide
     if (b->total == 0) return TIM_RT_OK;
     int rc;
     if (cfg.ray_sort != TIM_RT_SORT_NONE && (rc = batch_sort_scratch(c, b))) return rc;
-    int depth = wide ? b->wide_depth : b->depth;
-    if (cfg.stack_depth > depth) depth = cfg.stack_depth;
     uint32_t* err = static_cast<uint32_t*>(c->counters.ptr) + kErrWord;
-    TIMRT_CUDA(launch_multi(b->d_views, b->d_jobs, b->njobs, b->total, b->d_counter, err, depth, wide,
+    TIMRT_CUDA(launch_multi(b->d_views, b->d_jobs, b->njobs, b->total, b->d_counter, err, b->needs, wide,
                             cfg.ray_sort != TIM_RT_SORT_NONE ? &b->ss : nullptr, st, cfg));
     return TIM_RT_OK;
 }
@@ -1067,8 +1065,7 @@ int tim_rt_batch_create(tim_rt_ctx* c, const tim_rt_job* jobs, uint32_t num_jobs
             it = slot_of.emplace(J.scene, (uint32_t)views.size()).first;
             views.push_back(s->view);
             b->scene_ids.push_back(J.scene);
-            b->depth = std::max(b->depth, (int)s->depth);
-            b->wide_depth = std::max(b->wide_depth, (int)s->view.wide_depth);
+            b->needs.add_scene(s->view);
         }
         MultiJob m{};
         m.rays = J.d_rays;
@@ -1077,6 +1074,7 @@ int tim_rt_batch_create(tim_rt_ctx* c, const tim_rt_job* jobs, uint32_t num_jobs
         m.bary = reinterpret_cast<float2*>(J.d_bary);
         m.scene_slot = it->second;
         m.mode = J.mode;
+        b->needs.add_mode(J.mode);
         m.first = (uint32_t)total;
         m.n = J.n;
         for (int a = 0; a < 3; ++a) {

@@ -71,7 +71,7 @@ struct tim_rt_batch {
     DevBuf sort;                // ray-sort keys/values and radix-sort temporary storage
     std::vector<uint32_t> scene_ids;
     uint32_t njobs = 0, total = 0;
-    int depth = 1, wide_depth = 1;
+    MultiNeeds needs;
     bool wide = false;
     SceneView* d_views = nullptr;
     MultiJob* d_jobs = nullptr;

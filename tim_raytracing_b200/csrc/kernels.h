@@ -31,7 +31,7 @@ struct LaunchConfig {
 struct GridCache {
     static constexpr int kDevices = 64;
     std::mutex mu;
-    int blocks[kDevices][kStackSize + 9] = {};
+    int blocks[kDevices][kStackSize + 14] = {};   // k_walk: up to 13 words more a thread
     template <class F>
     int get(int depth, F compute) {
         int dev = 0;
@@ -114,10 +114,27 @@ struct SortScratch {
     size_t temp_bytes;
 };
 size_t multi_sort_temp_bytes(uint32_t total);
-// Resets `counter` and launches one persistent kernel over all jobs; with
-// cfg.ray_sort != 0 the rays are first ordered by the coherence key.
+// What the jobs of a batch need of the kernels: the deepest tree of each kind, whether
+// every scene has the binary form's trees (SceneView::nodes4), and the kinds of rays.
+struct MultiNeeds {
+    int depth = 1, wide_depth = 1, depth4 = 1;
+    bool four = true, any = false, closest = false;
+    void add_scene(const SceneView& v) {
+        depth = depth > (int)v.depth ? depth : (int)v.depth;
+        wide_depth = wide_depth > (int)v.wide_depth ? wide_depth : (int)v.wide_depth;
+        depth4 = depth4 > (int)v.depth4 ? depth4 : (int)v.depth4;
+        four = four && v.nodes4 != nullptr;
+    }
+    void add_mode(uint32_t mode) {
+        any = any || mode != TIM_RT_MODE_CLOSEST;
+        closest = closest || mode != TIM_RT_MODE_ANY;
+    }
+};
+// Resets `counter` (two words) and launches one persistent kernel over all jobs -- in the
+// binary form, where every scene has its trees, one for the closest-hit rays and one for
+// the any-hit rays; with cfg.ray_sort != 0 the rays are first ordered by the coherence key.
 cudaError_t launch_multi(const SceneView* views, const MultiJob* jobs, uint32_t njobs, uint32_t total, uint32_t* counter,
-                         uint32_t* err, int depth, bool wide, const SortScratch* sort, cudaStream_t stream,
+                         uint32_t* err, const MultiNeeds& needs, bool wide, const SortScratch* sort, cudaStream_t stream,
                          const LaunchConfig& cfg);
 
 // Light-probe update of probes [p0, p0 + np), nd directions each.

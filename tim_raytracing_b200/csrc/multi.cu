@@ -6,6 +6,7 @@
 #include "common.cuh"
 #include "trace_plain.cuh"
 #include "trace_wide.cuh"
+#include "walk.cuh"
 #include "kernels.h"
 #include "../../include/tim_rt.h"
 
@@ -161,6 +162,55 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 768 / BLOCK : 1) k_multi(const S
     }
 }
 
+// The rays of one kind of a batch, each on its scene's own trees (walk.cuh).
+struct MultiPolicy {
+    static constexpr bool kFilters = true, kManyScenes = true;
+    const SceneView* views;
+    const MultiJob* jobs;
+    uint32_t njobs;
+    const uint32_t* perm;
+    bool any;
+
+    __device__ __forceinline__ static bool is_any(const MultiJob& J, uint32_t i) {
+        return J.mode == TIM_RT_MODE_ANY ||
+               (J.mode == TIM_RT_MODE_PER_RAY && (__ldg(reinterpret_cast<const uint32_t*>(J.rays + i) + 7) & TIM_RT_RAY_ANY));
+    }
+    __device__ __forceinline__ bool keeps(uint32_t i) const {
+        const uint32_t item = perm ? __ldg(perm + i) : i;
+        const MultiJob& J = jobs[find_job(jobs, njobs, item)];
+        return is_any(J, item - J.first) == any;
+    }
+    __device__ __forceinline__ bool load(const SceneView&, uint32_t i, TravState& st) const {
+        const uint32_t item = perm ? __ldg(perm + i) : i;
+        st.slot = find_job(jobs, njobs, item);
+        const MultiJob& J = jobs[st.slot];
+        st.view = J.scene_slot;
+        st.slot2 = item - J.first;
+        const float4* rp = reinterpret_cast<const float4*>(J.rays + st.slot2);
+        const float4 a = __ldg(rp), b = __ldg(rp + 1);
+        st.r.ox = a.x; st.r.oy = a.y; st.r.oz = a.z;
+        st.r.dx = b.x; st.r.dy = b.y; st.r.dz = b.z;
+        st.t = a.w;
+        return true;
+    }
+    __device__ __forceinline__ void skip(uint32_t) const {}
+    __device__ __forceinline__ bool wants_nid(const TravState& st) const { return jobs[st.slot].nid != nullptr; }
+    __device__ __forceinline__ bool wants_bary(const TravState& st) const { return jobs[st.slot].bary != nullptr; }
+    __device__ __forceinline__ void store(const SceneView&, uint32_t, const TravState& st, float tmax) const {
+        const MultiJob& J = jobs[st.slot];
+        const uint32_t i = st.slot2;
+        if (st.any) {
+            J.hit[i] = make_uint4(st.hit ? 1u : 0u, 0u, 0u, __float_as_uint(tmax));
+            if (J.nid) J.nid[i] = 0xFFFFFFFFu;
+            if (J.bary) J.bary[i] = make_float2(0.f, 0.f);
+        } else {
+            J.hit[i] = make_uint4(st.rec0, st.rec1, st.rec2, __float_as_uint(st.t));
+            if (J.nid) J.nid[i] = st.hit ? st.nid : 0xFFFFFFFFu;
+            if (J.bary) J.bary[i] = make_float2(st.u, st.v);
+        }
+    }
+};
+
 template <int BLOCK, bool WIDE>
 static int grid_multi(int depth) {
     static GridCache cache;
@@ -197,8 +247,10 @@ size_t multi_sort_temp_bytes(uint32_t total) {
 }
 
 cudaError_t launch_multi(const SceneView* views, const MultiJob* jobs, uint32_t njobs, uint32_t total, uint32_t* counter,
-                         uint32_t* err, int depth, bool wide, const SortScratch* sort, cudaStream_t stream,
+                         uint32_t* err, const MultiNeeds& needs, bool wide, const SortScratch* sort, cudaStream_t stream,
                          const LaunchConfig& cfg) {
+    int depth = wide ? needs.wide_depth : needs.depth;
+    if (cfg.stack_depth > depth) depth = cfg.stack_depth;
     depth = depth < 1 ? 1 : (depth > kStackSize ? kStackSize : depth);
     const int refill = launch_knobs(cfg);
     const uint32_t* perm = nullptr;
@@ -215,7 +267,19 @@ cudaError_t launch_multi(const SceneView* views, const MultiJob* jobs, uint32_t 
         if (e != cudaSuccess) return e;
         perm = vb.Current();
     }
-    cudaMemsetAsync(counter, 0, 4, stream);
+    cudaMemsetAsync(counter, 0, 8, stream);
+    if (!wide && needs.four) {
+        SceneView v{};   // only the stacks' depths are taken from it
+        v.depth = (uint32_t)needs.depth;
+        v.depth4 = (uint32_t)needs.depth4;
+        MultiPolicy P{views, jobs, njobs, perm, false};
+        if (needs.closest) {
+            const cudaError_t e = launch_walk<false>(v, P, total, counter, err, stream, cfg, needs.any ? kPairFirst : kAlone);
+            if (e != cudaSuccess || !needs.any) return e;
+        }
+        P.any = true;
+        return launch_walk<true>(v, P, total, counter + 1, err, stream, cfg, needs.closest ? kPairSecond : kAlone);
+    }
     switch (cfg.block) {
         case 64:
             wide ? launch_multi_block<64, true>(views, jobs, njobs, total, perm, counter, err, depth, refill, stream)

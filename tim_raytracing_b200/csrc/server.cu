@@ -318,7 +318,7 @@ int issue_step(tim_rt_server* s, Plan& P) {
     SceneView* hv = static_cast<SceneView*>(sl.host);
     MultiJob* hj = reinterpret_cast<MultiJob*>(static_cast<uint8_t*>(sl.host) + round256(sizeof(SceneView) * maxj));
     std::map<Scene*, uint32_t> slot_of;
-    int depth = 1;
+    MultiNeeds needs;
     uint32_t total = 0, nj = 0;
     for (auto& ch : P.chunks) {
         Req* r = ch.first;
@@ -326,7 +326,7 @@ int issue_step(tim_rt_server* s, Plan& P) {
         if (it == slot_of.end()) {
             it = slot_of.emplace(r->scene, (uint32_t)slot_of.size()).first;
             hv[it->second] = r->scene->view;
-            depth = std::max(depth, s->wide ? (int)r->scene->view.wide_depth : (int)r->scene->depth);
+            needs.add_scene(r->scene->view);
         }
         MultiJob& J = hj[nj++];
         std::memset(&J, 0, sizeof(J));
@@ -336,6 +336,7 @@ int issue_step(tim_rt_server* s, Plan& P) {
         J.bary = r->d_bary ? r->d_bary + r->issued : nullptr;
         J.scene_slot = it->second;
         J.mode = r->r.mode;
+        needs.add_mode(J.mode);
         J.first = total;
         J.n = ch.second;
         total += ch.second;
@@ -356,10 +357,9 @@ int issue_step(tim_rt_server* s, Plan& P) {
     cfg.stats = nullptr;
     cfg.phase_ev = nullptr;
     cfg.ray_sort = TIM_RT_SORT_NONE;
-    if (cfg.stack_depth > depth) depth = cfg.stack_depth;
     uint32_t* err = static_cast<uint32_t*>(s->ctx->counters.ptr) + kErrWord;
     if (cudaEventRecord(sl.t_begin, s->comp) != cudaSuccess ||
-        launch_multi(sl.d_views, sl.d_jobs, nj, total, sl.d_counter, err, depth, s->wide, nullptr, s->comp, cfg) !=
+        launch_multi(sl.d_views, sl.d_jobs, nj, total, sl.d_counter, err, needs, s->wide, nullptr, s->comp, cfg) !=
             cudaSuccess ||
         cudaEventRecord(sl.t_end, s->comp) != cudaSuccess)
         return TIM_RT_EDEVICE;

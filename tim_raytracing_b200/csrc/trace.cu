@@ -18,8 +18,7 @@
 #include "common.cuh"
 #include "trace_plain.cuh"
 #include "trace_wide.cuh"
-#include "trace_any.cuh"
-#include "trace_pair.cuh"
+#include "walk.cuh"
 #include "kernels.h"
 #include "../../include/tim_rt.h"
 
@@ -64,19 +63,6 @@ template <class P, class = void>
 struct leaf_kind { static constexpr int value = kLeafOne; };
 template <class P>
 struct leaf_kind<P, decltype((void)P::kLeaf)> { static constexpr int value = P::kLeaf; };
-// Whether a policy wants its finished() hook called by the whole warp after each
-// round of stores.
-template <class P, class = void>
-struct finishes { static constexpr bool value = false; };
-template <class P>
-struct finishes<P, decltype((void)P::kFinishes)> { static constexpr bool value = P::kFinishes; };
-
-// Whether a policy traces only the items that keeps() tells of its batch.
-template <class P, class = void>
-struct filters { static constexpr bool value = false; };
-template <class P>
-struct filters<P, decltype((void)P::kFilters)> { static constexpr bool value = P::kFilters; };
-
 struct BatchPolicy {
     const tim_rt_ray* rays;
     uint4* hit;
@@ -107,8 +93,8 @@ struct BatchPolicy {
         }
     }
     __device__ __forceinline__ void skip(uint32_t) const {}
-    __device__ __forceinline__ bool wants_nid() const { return nid != nullptr; }
-    __device__ __forceinline__ bool wants_bary() const { return bary != nullptr; }
+    __device__ __forceinline__ bool wants_nid(const TravState&) const { return nid != nullptr; }
+    __device__ __forceinline__ bool wants_bary(const TravState&) const { return bary != nullptr; }
 };
 
 // The rays of one kind of a TIM_RT_MODE_PER_RAY batch: the two kinds walk different
@@ -181,8 +167,8 @@ struct CameraPolicy {
         out[2u * pix + 1u] = make_uint4(0u, 0u, 0u, 0u);
         leaf_nid[pix] = 0xFFFFFFFFu;
     }
-    __device__ __forceinline__ bool wants_nid() const { return true; }
-    __device__ __forceinline__ bool wants_bary() const { return false; }
+    __device__ __forceinline__ bool wants_nid(const TravState&) const { return true; }
+    __device__ __forceinline__ bool wants_bary(const TravState&) const { return false; }
 };
 
 // Secondary rays queued by band and kind (QueueBands). Segment e of the work items
@@ -279,58 +265,11 @@ struct SecondaryPolicy {
         }
     }
     __device__ __forceinline__ void skip(uint32_t) const {}
-    __device__ __forceinline__ bool wants_nid() const { return false; }
-    __device__ __forceinline__ bool wants_bary() const { return false; }
+    __device__ __forceinline__ bool wants_nid(const TravState&) const { return false; }
+    __device__ __forceinline__ bool wants_bary(const TravState&) const { return false; }
 };
 
 // -------------------------------------------------------------------- persistent loop
-
-// The work items of a launch: the policy's own count, or the launch's.
-template <class P, class = void>
-struct counts_items { static constexpr bool value = false; };
-template <class P>
-struct counts_items<P, decltype((void)&P::items)> { static constexpr bool value = true; };
-template <class Policy>
-__device__ __forceinline__ uint32_t items_of(const Policy& P, uint32_t n) {
-    if constexpr (counts_items<Policy>::value) return P.items();
-    else return n;
-}
-
-// Hands the items of a batch that a filtering policy (filters<Policy>) keeps to the
-// idle lanes of a warp: 32 items at a time are looked at, those kept wait in `pool`
-// (32 words of shared memory a warp) until lanes take them. start(item) is called by
-// the lanes that got one; sets exhausted once the batch is used up.
-template <class Policy, class Start>
-__device__ __forceinline__ void refill_filtered(const Policy& P, uint32_t n, uint32_t* counter, uint32_t* pool,
-                                                uint32_t need, uint32_t& used, uint32_t& have, bool& exhausted,
-                                                Start start) {
-    const uint32_t lane = threadIdx.x & 31u;
-    while (need) {
-        if (used == have) {
-            uint32_t base = 0;
-            if (lane == 0u) base = atomicAdd(counter, 32u);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base >= n) {
-                exhausted = true;
-                return;
-            }
-            const uint32_t item = base + lane;
-            const bool mine = item < n && P.keeps(item);
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine);
-            if (mine) pool[__popc(m & lanemask_lt())] = item;
-            __syncwarp();
-            used = 0;
-            have = (uint32_t)__popc(m);
-            continue;
-        }
-        const uint32_t r = (uint32_t)__popc(need & lanemask_lt());
-        const bool take = ((need >> lane) & 1u) && r < have - used;
-        if (take) start(pool[used + r]);
-        __syncwarp();
-        used = min(have, used + (uint32_t)__popc(need));
-        need &= ~__ballot_sync(0xFFFFFFFFu, take);
-    }
-}
 
 // sdepth: traversal-stack entries per thread (the tree depth; <= 32). The stack
 // lives in dynamic shared memory, entry k of thread t at [k * BLOCK + t].
@@ -420,102 +359,6 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
             pending = true;
         }
     }
-}
-
-// Rays of one kind on their own tree: any-hit rays on the 4-wide one (trace_any.cuh),
-// closest-hit rays on the binary one's child pairs (trace_pair.cuh). The same
-// persistent loop, with the ray's place in st.node alone -- an inner node, a leaf, or
-// kAnyIdle, which is also the lowest word of its stack, so that popping it ends the
-// walk. sdepth: stack words per thread; an any-hit ray that would need more takes the
-// plain binary walk, a closest-hit ray never does.
-//
-// A batch of both kinds is two launches (kPairFirst, kPairSecond) that may overlap: the
-// first lets the second start as soon as its own blocks leave room, so that the second's
-// rays fill the first's tail; neither reads what the other writes, and the second ends
-// only after the first has.
-constexpr int kAlone = 0, kPairFirst = 1, kPairSecond = 2;
-template <int BLOCK, bool ANY, class Policy>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_walk(SceneView s, Policy P, uint32_t n_static, uint32_t* counter,
-                                                              uint32_t* err, int sdepth, int knobs) {
-    extern __shared__ uint32_t stack_mem[];
-    // knobs: refill threshold (bits 0..7), phase-switch threshold (bits 8..15), role in a pair (bits 16..)
-    if ((knobs >> 16) == kPairFirst) cudaTriggerProgrammaticLaunchCompletion();
-    const int refill_min = knobs & 0xFF;
-    const uint32_t phase_sw = (uint32_t)(knobs >> 8) & 0xFFu;
-    uint32_t* stk = stack_mem + threadIdx.x;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = items_of(P, n_static);
-    uint32_t* org = stk + (size_t)sdepth * BLOCK;   // the ray's origin (any-hit) and direction
-    uint32_t* dir = org + 3 * BLOCK;
-    uint32_t* pool = stack_mem + (size_t)(sdepth + 6) * BLOCK + (threadIdx.x & ~31u);   // filters<Policy> only
-    uint32_t used = 0, have = 0;
-    const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(stk);
-    const uint32_t limit = bottom + ((uint32_t)sdepth - 5u) * BLOCK * 4u;   // an any-hit visit pushes up to four words
-
-    TravState st;
-    st.node = kAnyIdle;
-    bool pending = false, exhausted = false;
-    uint32_t idx = 0;
-    stk[0] = kAnyIdle;
-    auto start = [&](uint32_t item) {
-        idx = item;
-        if (P.load(s, idx, st)) {
-            if (ANY) any_init(s, st, bottom);
-            else pair_init(s, st, bottom);
-            if (ANY) put3<BLOCK>(org, st.r.ox, st.r.oy, st.r.oz);
-            put3<BLOCK>(dir, st.r.dx, st.r.dy, st.r.dz);
-            pending = true;
-        } else {
-            P.skip(idx);
-        }
-    };
-    for (;;) {
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, st.node == kAnyIdle);
-        if (idle && (exhausted || __popc(idle) >= refill_min || idle == 0xFFFFFFFFu)) {
-            const bool stored = pending && st.node == kAnyIdle;
-            if (stored) {
-                pending = false;
-                st.any = ANY;
-                if (ANY) get3<BLOCK>(org, st.r.ox, st.r.oy, st.r.oz);
-                get3<BLOCK>(dir, st.r.dx, st.r.dy, st.r.dz);
-                if (ANY) any_finish_or_walk(s, st, err);
-                else pair_finish(s, st, P.wants_nid(), P.wants_bary());
-                P.store(s, idx, st, st.t);   // an any-hit ray's t stays its tmax
-            }
-            if constexpr (finishes<Policy>::value) P.finished(stored, st.slot2);
-            if (exhausted) {
-                if (idle == 0xFFFFFFFFu) break;
-            } else if constexpr (filters<Policy>::value) {
-                refill_filtered(P, n, counter, pool, idle, used, have, exhausted, start);
-            } else {
-                const int leader = __ffs(idle) - 1;
-                uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(idle));
-                base = __shfl_sync(0xFFFFFFFFu, base, leader);
-                if ((uint64_t)base + (uint32_t)__popc(idle) >= n) exhausted = true;
-                const uint32_t my = base + __popc(idle & lanemask_lt());
-                if (((idle >> lane) & 1u) && my < n) start(my);
-            }
-        }
-        for (;;) {   // node rounds (see plain_step_warp)
-            const uint32_t nm = __ballot_sync(0xFFFFFFFFu, (int)st.node >= 0);
-            if (nm == 0u) break;
-            if ((uint32_t)__popc(nm) <= phase_sw &&
-                __any_sync(0xFFFFFFFFu, (int)st.node < 0 && st.node != kAnyIdle)) break;
-            if ((int)st.node >= 0) {
-                if (ANY) any_advance<BLOCK>(s, st, limit);
-                else pair_advance<BLOCK>(s, st, dir);
-            }
-        }
-        if ((int)st.node < 0 && st.node != kAnyIdle) {
-            Ray r{st.r.ox, st.r.oy, st.r.oz, 0.f, 0.f, 0.f};
-            if (ANY) get3<BLOCK>(org, r.ox, r.oy, r.oz);
-            get3<BLOCK>(dir, r.dx, r.dy, r.dz);
-            if (ANY) any_leaf<BLOCK>(s, st, r);
-            else pair_leaf<BLOCK>(s, st, r);
-        }
-    }
-    if ((knobs >> 16) == kPairSecond) cudaGridDependencySynchronize();
 }
 
 // -------------------------------------------------------------------- secondary ray generation
@@ -831,25 +674,6 @@ __global__ void __launch_bounds__(256) k_cull_lights(SceneView s, tim_rt_pass_da
 
 // -------------------------------------------------------------------- launchers
 
-// One word per stack entry, and a filtering policy's 32 words a warp of items not yet handed out.
-template <int BLOCK, class Policy>
-constexpr size_t stack_bytes(int depth) {
-    return sizeof(uint32_t) * (size_t)(depth + (filters<Policy>::value ? 1 : 0)) * BLOCK;
-}
-
-// Grid of a persistent kernel: as many resident blocks as the occupancy
-// calculator allows on every SM for this stack depth (cached per device and depth).
-template <int BLOCK, class Policy, class K>
-static int grid_of(GridCache& cache, K* kernel, int depth, int max_depth) {
-    return cache.get(depth, [=](int dev) {
-        int sms = 0, per = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stack_bytes<BLOCK, Policy>(max_depth));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, BLOCK, stack_bytes<BLOCK, Policy>(depth));
-        return (sms > 0 ? sms : 1) * (per > 0 ? per : 1);
-    });
-}
-
 template <int BLOCK, bool WIDE, bool STATS, class Policy>
 static void launch_block(const SceneView& s, const Policy& P, uint32_t n_static,
                          uint32_t* counter, uint32_t* err, unsigned long long* stats, int depth, int refill,
@@ -877,57 +701,6 @@ static cudaError_t launch_persistent(const SceneView& s, const Policy& P, uint32
         default: launch_block<128, WIDE, false>(s, P, n_static, counter, err, nullptr, depth, refill, stream); break;
     }
     return cudaGetLastError();
-}
-
-// Most stack words of an any-hit and a closest-hit ray of k_walk. 24 against 16 words:
-// the frame's any-hit rays the same, those of a probe update in 1M triangles 1.60
-// against 2.01 ms (16 overflow often enough there for the binary walk to show).
-constexpr int kAnyStack = 24, kWalkStack = kStackSize + 2;
-
-template <int BLOCK, bool ANY, class Policy>
-static cudaError_t launch_walk_block(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter,
-                                     uint32_t* err, int depth, int knobs, int role, int share, cudaStream_t stream) {
-    static GridCache cache;
-    const int words = depth + 6;   // and the ray's origin and direction
-    const int grid = grid_of<BLOCK, Policy>(cache, k_walk<BLOCK, ANY, Policy>, words, kWalkStack + 6);
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(share > 1 && grid >= share ? grid / share : grid);
-    lc.blockDim = dim3(BLOCK);
-    lc.dynamicSmemBytes = stack_bytes<BLOCK, Policy>(words);
-    lc.stream = stream;
-    cudaLaunchAttribute at{};
-    if (role == kPairSecond) {
-        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at.val.programmaticStreamSerializationAllowed = 1;
-        lc.attrs = &at;
-        lc.numAttrs = 1;
-    }
-    return cudaLaunchKernelEx(&lc, k_walk<BLOCK, ANY, Policy>, s, P, n_static, counter, err, depth, knobs | role << 16);
-}
-
-// One launch of k_walk, or one of a pair (of which the first may be given a share of the
-// GPU only). Stack words: a closest-hit ray leaves one child a level waiting, an any-hit
-// ray up to three slots, of which kAnyStack words are kept; the end marker; and the word
-// above the top, which a push writes whether it keeps it or not.
-template <bool ANY, class Policy>
-static cudaError_t launch_walk(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter, uint32_t* err,
-                               cudaStream_t stream, const LaunchConfig& cfg, int role = kAlone, int share = 1) {
-    int depth = (int)s.depth + 2;
-    LaunchConfig c = cfg;
-    if (ANY) {
-        depth = 3 * (int)s.depth4 + 2;
-        depth = depth < 6 ? 6 : (depth > kAnyStack ? kAnyStack : depth);
-        // any-hit rays of one origin's neighbourhood profit more from starting together (they
-        // read the same nodes; the L1 binds this walk): 16 -> 24 idle lanes, 0.81 -> 0.73 ms
-        // for the 5.1M any-hit rays of the 1080p frame. launch_knobs limits it to 32.
-        c.refill_min = cfg.refill_min + cfg.refill_min / 2;
-    }
-    const int knobs = launch_knobs(c);
-    switch (cfg.block) {
-        case 64: return launch_walk_block<64, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
-        case 256: return launch_walk_block<256, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
-        default: return launch_walk_block<128, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
-    }
 }
 
 // Launches of the binary form take the two trees where the scene has them; the
@@ -1164,8 +937,8 @@ struct ProbePolicy {
         leaf_nid[st.slot] = st.hit ? st.nid : 0xFFFFFFFFu;
     }
     __device__ __forceinline__ void skip(uint32_t) const {}
-    __device__ __forceinline__ bool wants_nid() const { return true; }
-    __device__ __forceinline__ bool wants_bary() const { return false; }
+    __device__ __forceinline__ bool wants_nid(const TravState&) const { return true; }
+    __device__ __forceinline__ bool wants_bary(const TravState&) const { return false; }
 };
 
 // Shadow rays of the probe hits: the sun (tmax = TMAX) and the hit leaf's lights

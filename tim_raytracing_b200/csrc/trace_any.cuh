@@ -101,6 +101,7 @@ __device__ __forceinline__ void any_init(const SceneView& s, TravState& st, uint
     st.px = base + (st.ix < 0.0f ? 32u : 0u);
     st.py = base + (st.iy < 0.0f ? 96u : 64u);
     st.pz = base + (st.iz < 0.0f ? 160u : 128u);
+    st.refs = base + 192u;
     const float fx = fabsf(ux), fy = fabsf(uy), fz = fabsf(uz);
     bool ok = max3_nan(fx, fy, fz) <= dhi && max3_nan(fabsf(st.r.ox), fabsf(st.r.oy), fabsf(st.r.oz)) <= ohi && st.t == st.t;
     if (!(min3_nan(fx, fy, fz) >= dlo)) {   // a zero component, or one too small
@@ -157,11 +158,16 @@ __device__ __forceinline__ void get3(const uint32_t* p, float& x, float& y, floa
     z = __uint_as_float(p[2 * BLOCK]);
 }
 
+// The references of node 0.
+__device__ __forceinline__ const char* four_refs(const SceneView& s) {
+    return reinterpret_cast<const char*>(s.nodes4) + 192u;
+}
+
 // One advance of one lane from the inner node st.node: its slots whose boxes are
 // entered go onto the stack, smallest box first, and the last one is taken. (The
 // entered box nearest first instead: 6 % fewer visits, but 20 more instructions each.)
 template <int BLOCK>
-__device__ __forceinline__ void any_advance(const SceneView& s, TravState& st, uint32_t limit) {
+__device__ __forceinline__ void any_advance(TravState& st, const char* refs_base, uint32_t limit) {
     if (st.top > limit) {   // more slots wait than the stack has room for: the binary walk
         st.leaf = 1u;
         st.node = kAnyIdle;
@@ -172,7 +178,7 @@ __device__ __forceinline__ void any_advance(const SceneView& s, TravState& st, u
     load8(st.px + off, nx, fx);
     load8(st.py + off, ny, fy);
     load8(st.pz + off, nz, fz);
-    const uint4 ref = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(s.nodes4) + off + 192u));
+    const uint4 ref = __ldg(reinterpret_cast<const uint4*>(refs_base + off));
     const float nxs[4] = {nx.x, nx.y, nx.z, nx.w}, nys[4] = {ny.x, ny.y, ny.z, ny.w}, nzs[4] = {nz.x, nz.y, nz.z, nz.w};
     const float fxs[4] = {fx.x, fx.y, fx.z, fx.w}, fys[4] = {fy.x, fy.y, fy.z, fy.w}, fzs[4] = {fz.x, fz.y, fz.z, fz.w};
     const uint32_t refs[4] = {ref.x, ref.y, ref.z, ref.w};
@@ -196,24 +202,25 @@ __device__ __forceinline__ uint32_t leaf_ref(const SceneView& s, uint32_t ref, u
     return cnt;
 }
 
-// Tests a leaf's triangles in their stored order (bvh_collide_fast,
-// bvhCollision.glsl:241-284); a hit ends the walk, otherwise the next slot is taken.
-template <int BLOCK>
-__device__ __forceinline__ void any_leaf(const SceneView& s, TravState& st, const Ray& r) {
-    uint32_t first;
-    const uint32_t cnt = leaf_ref(s, st.node, first);
-    const float4* tp = s.ptris + 3u * first;
+// A leaf's triangles in their stored order on the ray's own lane: an any-hit ray's first
+// hit (bvh_collide_fast, bvhCollision.glsl:241-284; returns true), or every hit of a
+// closest-hit ray below t, which it shrinks to 1e-5 under the hit (bvh_collide,
+// bvhCollision.glsl:177-239).
+template <bool ANY>
+__device__ __forceinline__ bool leaf_triangles(const float4* ptris, TravState& st, const Ray& r, uint32_t first, uint32_t cnt) {
+    const float4* tp = ptris + 3ull * first;
     for (uint32_t i = 0; i < cnt; ++i, tp += 3) {
         const float4 A = __ldg(tp), B = __ldg(tp + 1), C = __ldg(tp + 2);
         float u, v;
-        if (collide_triangle_e(r, A.x, A.y, A.z, B.x, B.y, B.z, C.x, C.y, C.z, st.t, u, v) > 0.0f) {
-            st.hit = true;
-            st.node = kAnyIdle;
+        const float t = collide_triangle_e(r, A.x, A.y, A.z, B.x, B.y, B.z, C.x, C.y, C.z, st.t, u, v);
+        if (t > 0.0f) {
             st.nid = first + i;
-            return;
+            if (ANY) return true;
+            st.t = t - kOffsetRayCollision;
+            st.hit = true;
         }
     }
-    st.node = stack_pop<BLOCK>(st.top);
+    return false;
 }
 
 // Whether the ray's answer stands (see the header): no hit, or a hit in a leaf that

@@ -58,10 +58,14 @@ __device__ __forceinline__ void pair_init(const SceneView& s, TravState& st, uin
     st.px = base + (__float_as_uint(st.r.dx) >> 31 << 4);
     st.py = base + 32u + (__float_as_uint(st.r.dy) >> 31 << 4);
     st.pz = base + 64u + (__float_as_uint(st.r.dz) >> 31 << 4);
+    st.refs = base + 96u;
     st.top = bottom;
     st.hit = false;
     st.node = s.root_pair;
 }
+
+// The references of record 0.
+__device__ __forceinline__ const char* pair_refs(const SceneView& s) { return reinterpret_cast<const char*>(s.pairs) + 96u; }
 
 // The slab values of one axis of both children.
 __device__ __forceinline__ void pair_slab(float2 p, float o, float inv, float& t0, float& t1) {
@@ -79,12 +83,12 @@ static __device__ __noinline__ PairOpen pair_exact(Ray r, float2 nx, float2 fx, 
 
 // One advance of one lane from record st.node (see plain_advance).
 template <int BLOCK>
-__device__ __forceinline__ void pair_advance(const SceneView& s, TravState& st, const uint32_t* dir) {
+__device__ __forceinline__ void pair_advance(TravState& st, const char* refs, const uint32_t* dir) {
     const uint64_t off = (uint64_t)st.node * kPairBytes;
     const float4 X = __ldg(reinterpret_cast<const float4*>(st.px + off));
     const float4 Y = __ldg(reinterpret_cast<const float4*>(st.py + off));
     const float4 Z = __ldg(reinterpret_cast<const float4*>(st.pz + off));
-    const uint2 ref = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(s.pairs) + off + 96u));
+    const uint2 ref = __ldg(reinterpret_cast<const uint2*>(refs + off));
     const uint32_t r0 = ref.x, r1 = ref.y;
     const float2 nx = make_float2(X.x, X.y), fx = make_float2(X.z, X.w);
     const float2 ny = make_float2(Y.x, Y.y), fy = make_float2(Y.z, Y.w);
@@ -125,25 +129,6 @@ __device__ __forceinline__ void pair_advance(const SceneView& s, TravState& st, 
     stack_push<BLOCK>(st.top, first1 ? r0 : r1, both);
     if (h0 || h1) st.node = take1 ? r1 : r0;
     else st.node = stack_pop<BLOCK>(st.top);
-}
-
-// Leaf visit (bvh_collide, bvhCollision.glsl:177-239): every hit below t shrinks t by 1e-5 under it.
-template <int BLOCK>
-__device__ __forceinline__ void pair_leaf(const SceneView& s, TravState& st, const Ray& r) {
-    uint32_t first;
-    const uint32_t cnt = leaf_ref(s, st.node, first);
-    const float4* tp = s.ptris + 3u * first;
-    for (uint32_t i = 0; i < cnt; ++i, tp += 3) {
-        const float4 A = __ldg(tp), B = __ldg(tp + 1), C = __ldg(tp + 2);
-        float u, v;
-        const float t = collide_triangle_e(r, A.x, A.y, A.z, B.x, B.y, B.z, C.x, C.y, C.z, st.t, u, v);
-        if (t > 0.0f) {
-            st.t = t - kOffsetRayCollision;
-            st.nid = first + i;
-            st.hit = true;
-        }
-    }
-    st.node = stack_pop<BLOCK>(st.top);
 }
 
 // The outputs of a ray whose walk is over: the hit triangle's record words, its leaf's

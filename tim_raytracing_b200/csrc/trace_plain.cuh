@@ -46,6 +46,8 @@ struct TravState {
     // planes per axis
     float anx, any_, anz, afx, afy, afz;
     const char *px, *py, *pz;   // where the ray reads an axis' planes, for node 0
+    const char* refs;           // the references of node 0 (batched launches: each ray its scene's)
+    uint32_t view;              // batched launches: the ray's scene
     uint32_t top;               // shared-memory address of the stack's top word
     uint32_t* err;      // two-level walk: the device error word (a nested walk's stack guard)
 };
