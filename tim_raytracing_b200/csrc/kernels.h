@@ -78,12 +78,13 @@ struct CameraBands {
 // [0] pixel work, [1] secondary work, [2, 2 + 26 nb) per-band per-kind counts,
 // [2 + 26 nb, 3 + 52 nb) their prefix (the last entry = secondary rays traced),
 // [3 + 52 nb, 3 + 53 nb) finished rays per band, [3 + 53 nb, 3 + 54 nb) rays per band,
-// [3 + 54 nb] closest-hit secondary work (a launch of its own with the 4-wide tree).
+// [3 + 54 nb] closest-hit secondary work (a launch of its own with the 4-wide tree),
+// [4 + 54 nb] generator blocks done.
 uint32_t camera_queue_kinds();
 // Queue segments of a probe update (np*nd slots each): the sun and the 16 light
 // slots, the only kinds its shadow-ray generator emits.
 uint32_t probe_queue_kinds();
-constexpr uint32_t cam_counter_words(uint32_t nb) { return 4u + 54u * nb; }
+constexpr uint32_t cam_counter_words(uint32_t nb) { return 5u + 54u * nb; }
 constexpr uint32_t kCamCounterWords = cam_counter_words(1), kCamTotalWord = 54;
 cudaError_t launch_camera(const SceneView& s, const tim_rt_pass_data& pd, uint32_t flags, uint32_t seed,
                           const uint32_t* tile_counts, const uint32_t* tile_lists, uint32_t* out, uint32_t* bounce_out,

@@ -23,7 +23,7 @@ namespace {
 
 constexpr uint32_t kMaxPix = TIM_RT_NOALLOC_MAX_PIXELS;
 constexpr uint32_t kKinds = 26;                 // secondary-ray kinds of the camera pipeline
-constexpr uint32_t kHeaderWords = 128;          // counters [0, 55), error word [64]
+constexpr uint32_t kHeaderWords = 128;          // counters [0, 59), error word [64]
 constexpr uint32_t kNidWords = kMaxPix;
 constexpr uint32_t kPixelWords = kKinds * kMaxPix;
 constexpr uint32_t kRayWords = kKinds * kMaxPix * 8u;
