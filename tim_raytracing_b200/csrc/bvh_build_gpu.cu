@@ -295,6 +295,28 @@ __global__ void k_sah_cost(uint32_t n, uint32_t max_leaf, float ci_, float ct, c
     }
 }
 
+// The 127 subsets of a treelet's leaves by size (as many leaves as the size, in
+// ascending order), and where each size starts.
+struct SubsetTable {
+    uint8_t set[kSubsets];
+    uint8_t start[kTreeletLeaves + 2];
+};
+constexpr SubsetTable subset_table() {
+    SubsetTable t{};
+    uint32_t at = 0;
+    for (int k = 0; k <= kTreeletLeaves; ++k) {
+        t.start[k] = (uint8_t)at;
+        for (int sub = 0; sub < kSubsets; ++sub) {
+            int bits = 0;
+            for (int i = 0; i < kTreeletLeaves; ++i) bits += (sub >> i) & 1;
+            if (bits == k) t.set[at++] = (uint8_t)sub;
+        }
+    }
+    t.start[kTreeletLeaves + 1] = (uint8_t)at;
+    return t;
+}
+__constant__ SubsetTable c_subsets = subset_table();
+
 // One treelet pass, a warp per treelet: every lane walks from one radix leaf up
 // to the root; the lane that arrives second at a node has the treelet rooted
 // there to restructure, and the warp takes its lanes' treelets one after another,
@@ -302,17 +324,32 @@ __global__ void k_sah_cost(uint32_t n, uint32_t max_leaf, float ci_, float ct, c
 // treelet root is final by then (its subtree's walks have all passed), so the
 // warp owns the treelet; writes are fenced before the next arrival, reads of
 // other warps' writes bypass L1.
+//
+// What bounds it: the chain of a treelet's loads (a treelet opens five nodes, each found
+// by the one before) and the instructions of its programme. So lane i holds leaf i of the
+// treelet with its children's ids, which costs one round trip an opening; a size's subsets
+// go to consecutive lanes (taken in numeric order, a lane skipping the other sizes, the
+// programme took three times the rounds); the rebuilt nodes are written a lane each.
+// 300K triangles: 1.25 -> 0.68 ms a pass, 460 -> 256 M instructions.
 __global__ void __launch_bounds__(kTreeletWarps * 32) k_treelet(uint32_t n, uint32_t max_leaf, float ci_, float ct,
                                                                 uint32_t* left, uint32_t* right, uint32_t* parent,
                                                                 Aabb* box, float* cost, uint32_t* size, uint8_t* coll,
                                                                 uint32_t* arrive) {
-    __shared__ float s_area_all[kTreeletWarps][kSubsets];
-    __shared__ float s_cost_all[kTreeletWarps][kSubsets];
-    __shared__ uint8_t s_part_all[kTreeletWarps][kSubsets];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    float* s_area = s_area_all[w];
-    float* s_cost = s_cost_all[w];
-    uint8_t* s_part = s_part_all[w];
+    struct Warp {
+        float area[kSubsets], cost[kSubsets];
+        uint8_t part[kSubsets];
+        Aabb box[kTreeletLeaves];
+        float leaf_cost[kTreeletLeaves];
+        uint32_t leaf[kTreeletLeaves], leaf_size[kTreeletLeaves], inner[kTreeletLeaves - 2];
+        uint32_t node[kTreeletLeaves - 1], set[kTreeletLeaves - 1], kid[kTreeletLeaves - 1][2];   // the rebuilt nodes
+    };
+    __shared__ Warp warps[kTreeletWarps];
+    __shared__ uint8_t subsets[kSubsets];
+    static_assert(kTreeletWarps * 32 == kSubsets, "one table entry a thread");
+    const uint32_t lane = threadIdx.x & 31u;
+    Warp& W = warps[threadIdx.x >> 5];
+    subsets[threadIdx.x] = c_subsets.set[threadIdx.x];
+    __syncthreads();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;   // radix leaf j: handle n - 1 + j
     bool active = j < n;
     uint32_t cur = n - 1u + j;
@@ -345,60 +382,70 @@ __global__ void __launch_bounds__(kTreeletWarps * 32) k_treelet(uint32_t n, uint
             const int src = __ffs(todo) - 1;
             todo &= todo - 1u;
             const uint32_t root = __shfl_sync(0xFFFFFFFFu, p, src);
-            // the treelet below root (every lane forms it, from the same loads):
-            // open the largest-area internal node until 7 leaves
-            uint32_t leaf[kTreeletLeaves], inner[kTreeletLeaves - 2];
-            Aabb lb[kTreeletLeaves];
-            float la[kTreeletLeaves];   // area of an internal leaf of the treelet, -1 for a triangle
-            int nl = 2, ni = 0;
-            leaf[0] = __ldcg(left + root);
-            leaf[1] = __ldcg(right + root);
-            lb[0] = load_box_cg(box + leaf[0]);
-            lb[1] = load_box_cg(box + leaf[1]);
-            la[0] = leaf[0] >= n - 1u ? -1.0f : half_area(lb[0]);
-            la[1] = leaf[1] >= n - 1u ? -1.0f : half_area(lb[1]);
+            // the treelet below root, leaf i on lane i: open the largest-area internal
+            // node (the first of equals) until 7 leaves
+            uint32_t my = 0, my_left = 0, my_right = 0, my_size = 0;
+            float my_cost = 0.f;
+            Aabb my_box;
+            uint32_t key = 0;   // orders like the area; 0 for a triangle and for lanes without a leaf
+            auto take = [&](uint32_t x) {
+                my = x;
+                my_box = load_box_cg(box + x);
+                my_size = __ldcg(size + x);
+                my_cost = __ldcg(cost + x);
+                key = 0;
+                if (x < n - 1u) {
+                    my_left = __ldcg(left + x);
+                    my_right = __ldcg(right + x);
+                    const float a = half_area(my_box);
+                    key = a >= 0.0f ? __float_as_uint(fabsf(a)) + 1u : 0u;
+                }
+            };
+            if (lane < 2u) take(__ldcg((lane ? right : left) + root));
+            int nl = 2;
+            uint32_t opened = 0;
             while (nl < kTreeletLeaves) {
-                int best = -1;
-                float ba = -1.0f;
-                for (int i = 0; i < nl; ++i)
-                    if (la[i] > ba) { ba = la[i]; best = i; }
-                if (best < 0) break;
-                const uint32_t x = leaf[best];
-                inner[ni++] = x;
-                leaf[best] = __ldcg(left + x);
-                leaf[nl] = __ldcg(right + x);
-                lb[best] = load_box_cg(box + leaf[best]);
-                lb[nl] = load_box_cg(box + leaf[nl]);
-                la[best] = leaf[best] >= n - 1u ? -1.0f : half_area(lb[best]);
-                la[nl] = leaf[nl] >= n - 1u ? -1.0f : half_area(lb[nl]);
+                const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, key);
+                if (most == 0u) break;
+                const int best = __ffs(__ballot_sync(0xFFFFFFFFu, key == most)) - 1;
+                const uint32_t x = __shfl_sync(0xFFFFFFFFu, my, best), xl = __shfl_sync(0xFFFFFFFFu, my_left, best),
+                               xr = __shfl_sync(0xFFFFFFFFu, my_right, best);
+                if (lane == (uint32_t)nl - 2u) opened = x;
+                if ((int)lane == best || (int)lane == nl) take((int)lane == best ? xl : xr);
                 ++nl;
             }
             if (nl < 3) continue;   // two triangles: nothing to rearrange
-            uint32_t lsz[kTreeletLeaves];
-            float lcost[kTreeletLeaves];
-#pragma unroll
-            for (int i = 0; i < kTreeletLeaves; ++i) {
-                lsz[i] = i < nl ? __ldcg(size + leaf[i]) : 0u;
-                lcost[i] = i < nl ? __ldcg(cost + leaf[i]) : 0.f;
+            if ((int)lane < nl) {
+                W.leaf[lane] = my;
+                W.box[lane] = my_box;
+                W.leaf_size[lane] = my_size;
+                W.leaf_cost[lane] = my_cost;
+                if ((int)lane < nl - 2) W.inner[lane] = opened;
             }
+            __syncwarp();
+            // the box and the triangles of a subset of the leaves
+            auto unite = [&](uint32_t sub, uint32_t& cnt) {
+                Aabb u;
+                for (int k = 0; k < 3; ++k) { u.lo[k] = INFINITY; u.hi[k] = -INFINITY; }
+                cnt = 0;
+                for (uint32_t m = sub; m; m &= m - 1u) {
+                    const uint32_t i = (uint32_t)__ffs(m) - 1u;
+                    u = merge_box(u, W.box[i]);
+                    cnt += W.leaf_size[i];
+                }
+                return u;
+            };
             // area of every subset of the treelet's leaves; a single leaf keeps its
             // cost, a larger subset starts at its cost as one leaf (if small enough)
             const uint32_t full = (1u << nl) - 1u;
-            for (uint32_t sub = lane + 1u; sub <= full; sub += 32u) {
-                Aabb u;
-                for (int k = 0; k < 3; ++k) { u.lo[k] = INFINITY; u.hi[k] = -INFINITY; }
-                uint32_t cnt = 0;
-                float single = 0.f;
-#pragma unroll
-                for (int i = 0; i < kTreeletLeaves; ++i)
-                    if (sub & (1u << i)) {
-                        u = merge_box(u, lb[i]);
-                        cnt += lsz[i];
-                        single = lcost[i];
-                    }
-                const float a = half_area(u);
-                s_area[sub] = a;
-                s_cost[sub] = (sub & (sub - 1u)) == 0u ? single : (cnt <= max_leaf ? ct * a * (float)cnt : INFINITY);
+            for (uint32_t at = 1u + lane; at < (uint32_t)kSubsets; at += 32u) {
+                const uint32_t sub = subsets[at];
+                if (sub & ~full) continue;
+                uint32_t cnt;
+                const float a = half_area(unite(sub, cnt));
+                W.area[sub] = a;
+                W.cost[sub] = (sub & (sub - 1u)) == 0u ? W.leaf_cost[__ffs(sub) - 1]
+                                                       : (cnt <= max_leaf ? ct * a * (float)cnt : INFINITY);
             }
             __syncwarp();
             // best split of every subset, by size: all proper subsets are done first.
@@ -415,14 +462,15 @@ __global__ void __launch_bounds__(kTreeletWarps * 32) k_treelet(uint32_t n, uint
                     const uint32_t sub = k == nl ? full : (real ? full ^ (1u << gi) : full);
                     const uint32_t low = sub & (0u - sub), rest = sub ^ low;
                     const uint32_t nsplit = (1u << (k - 1)) - 1u;   // subsets q of rest but rest itself
+                    // the j-th subset of rest: sub misses at most one leaf, so rest is the leaves
+                    // above its lowest but for one, and j's bits move up past that one
+                    const uint32_t shift = (uint32_t)__ffs(rest) - 1u, hole = ((rest >> shift) + 1u) & ~(rest >> shift);
                     float best = INFINITY;
                     uint32_t bp = 0xFFu;
                     for (uint32_t j = gl; real && j < nsplit; j += G) {
-                        uint32_t q = 0, jj = j;   // the j-th subset of rest: j's bits on rest's bits
-                        for (uint32_t b = rest; b; b &= b - 1u, jj >>= 1)
-                            if (jj & 1u) q |= b & (0u - b);
+                        const uint32_t q = ((j & (hole - 1u)) | ((j & ~(hole - 1u)) << 1)) << shift;
                         const uint32_t P = q | low;
-                        const float c = s_cost[P] + s_cost[sub ^ P];
+                        const float c = W.cost[P] + W.cost[sub ^ P];
                         if (c < best || (c == best && P < bp)) { best = c; bp = P; }
                     }
                     for (uint32_t o = G >> 1; o; o >>= 1) {   // least cost in the group, ties to the lower split
@@ -431,75 +479,75 @@ __global__ void __launch_bounds__(kTreeletWarps * 32) k_treelet(uint32_t n, uint
                         if (ob < best || (ob == best && op < bp)) { best = ob; bp = op; }
                     }
                     if (real && gl == 0u) {
-                        const float ci = ci_ * s_area[sub] + best;
-                        const float cl = s_cost[sub];
-                        s_cost[sub] = fminf(cl, ci);
-                        s_part[sub] = (uint8_t)(bp == 0xFFu ? low : bp) | (cl <= ci ? kCollapse : 0u);
+                        const float ci = ci_ * W.area[sub] + best;
+                        const float cl = W.cost[sub];
+                        W.cost[sub] = fminf(cl, ci);
+                        W.part[sub] = (uint8_t)(bp == 0xFFu ? low : bp) | (cl <= ci ? kCollapse : 0u);
                     }
                     __syncwarp();
                     continue;
                 }
-                for (uint32_t sub = lane + 1u; sub <= full; sub += 32u) {
-                    if (__popc(sub) != k) continue;
+                for (uint32_t at = c_subsets.start[k] + lane; at < c_subsets.start[k + 1]; at += 32u) {
+                    const uint32_t sub = subsets[at];
+                    if (sub & ~full) continue;
                     const uint32_t low = sub & (0u - sub), rest = sub ^ low;
                     float best = INFINITY;
                     uint32_t bp = low;
-                    for (uint32_t q = rest;; q = (q - 1u) & rest) {
+                    for (uint32_t q = (rest - 1u) & rest;; q = (q - 1u) & rest) {   // rest itself is no split
                         const uint32_t P = q | low;
-                        if (P != sub) {
-                            const float c = s_cost[P] + s_cost[sub ^ P];
-                            if (c < best) { best = c; bp = P; }
-                        }
+                        const float c = W.cost[P] + W.cost[sub ^ P];
+                        if (c < best) { best = c; bp = P; }
                         if (q == 0u) break;
                     }
-                    const float ci = ci_ * s_area[sub] + best;
-                    const float cl = s_cost[sub];
-                    s_cost[sub] = fminf(cl, ci);
-                    s_part[sub] = (uint8_t)bp | (cl <= ci ? kCollapse : 0u);
+                    const float ci = ci_ * W.area[sub] + best;
+                    const float cl = W.cost[sub];
+                    W.cost[sub] = fminf(cl, ci);
+                    W.part[sub] = (uint8_t)bp | (cl <= ci ? kCollapse : 0u);
                 }
                 __syncwarp();
             }
-            // rebuild (lane 0): root keeps its place; the other internal nodes are
-            // reused in order. A subset that becomes one leaf still gets its best
-            // split below it, so its triangles stay reachable from it.
+            // rebuild: root keeps its place; the other internal nodes are reused in
+            // order. A subset that becomes one leaf still gets its best split below it,
+            // so its triangles stay reachable from it. Lane 0 lays the links out, then
+            // each rebuilt node is a lane's to write.
             if (lane == 0u) {
                 uint32_t stk_node[kTreeletLeaves], stk_set[kTreeletLeaves];
-                int sp = 0, next = 0;
+                int sp = 0, next = 0, done = 0;
                 stk_node[sp] = root;
                 stk_set[sp++] = full;
                 while (sp > 0) {
                     --sp;
                     const uint32_t node = stk_node[sp], set = stk_set[sp];
-                    const uint8_t part = s_part[set];
-                    const uint32_t P = part & (kCollapse - 1u), Q = set ^ P;
-                    uint32_t kid[2];
-                    const uint32_t sides[2] = {P, Q};
+                    const uint32_t P = W.part[set] & (kCollapse - 1u);
+                    W.node[done] = node;
+                    W.set[done] = set;
                     for (int k = 0; k < 2; ++k) {
-                        if ((sides[k] & (sides[k] - 1u)) == 0u) {
-                            kid[k] = leaf[__ffs(sides[k]) - 1];
+                        const uint32_t side = k ? set ^ P : P;
+                        uint32_t kid;
+                        if ((side & (side - 1u)) == 0u) {
+                            kid = W.leaf[__ffs(side) - 1];
                         } else {
-                            kid[k] = inner[next++];
-                            stk_node[sp] = kid[k];
-                            stk_set[sp++] = sides[k];
+                            kid = W.inner[next++];
+                            stk_node[sp] = kid;
+                            stk_set[sp++] = side;
                         }
-                        parent[kid[k]] = node;
+                        W.kid[done][k] = kid;
                     }
-                    left[node] = kid[0];
-                    right[node] = kid[1];
-                    Aabb u;
-                    for (int k = 0; k < 3; ++k) { u.lo[k] = INFINITY; u.hi[k] = -INFINITY; }
-                    uint32_t cnt = 0;
-#pragma unroll
-                    for (int i = 0; i < kTreeletLeaves; ++i)
-                        if (set & (1u << i)) {
-                            u = merge_box(u, lb[i]);
-                            cnt += lsz[i];
-                        }
-                    box[node] = u;
-                    size[node] = cnt;
-                    coll[node] = (part & kCollapse) ? 1u : 0u;
-                    cost[node] = s_cost[set];
+                    ++done;
                 }
+            }
+            __syncwarp();
+            if ((int)lane < nl - 1) {
+                const uint32_t node = W.node[lane], set = W.set[lane], l = W.kid[lane][0], r = W.kid[lane][1];
+                parent[l] = node;
+                parent[r] = node;
+                left[node] = l;
+                right[node] = r;
+                uint32_t cnt;
+                box[node] = unite(set, cnt);
+                size[node] = cnt;
+                coll[node] = (W.part[set] & kCollapse) ? 1u : 0u;
+                cost[node] = W.cost[set];
                 __threadfence();
             }
             __syncwarp();
