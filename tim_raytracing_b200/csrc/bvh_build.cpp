@@ -18,7 +18,7 @@
 using namespace timrt;
 
 struct tim_rt_bvh_blob {
-    std::vector<uint8_t> bytes;
+    timrt::RawVec<uint8_t> bytes;
     uint32_t ranges[7][2];
     tim_rt_push_constants pc;
     float aabb[6];

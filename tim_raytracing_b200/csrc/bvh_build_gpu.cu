@@ -29,6 +29,7 @@
 // Trees deeper than max_depth (the reference's traversal keeps a 32-bit
 // bitstack) are refused with TIM_RT_EUNSUPPORTED.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <cub/cub.cuh>
 #include <algorithm>
 #include <cstring>
@@ -38,7 +39,7 @@
 #include "context.h"
 
 struct tim_rt_bvh_blob {   // same definition as bvh_build.cpp
-    std::vector<uint8_t> bytes;
+    timrt::RawVec<uint8_t> bytes;
     uint32_t ranges[7][2];
     tim_rt_push_constants pc;
     float aabb[6];
@@ -968,8 +969,19 @@ int tim_rt_build_bvh_gpu(tim_rt_ctx* c, const float* pos, uint32_t num_vertex, c
     place(TIM_RT_RANGE_NODE, 64u * num_nodes);
     blob->ranges[TIM_RT_RANGE_LEAF][0] = off;
     blob->ranges[TIM_RT_RANGE_LEAF][1] = 4u * leaf_words;
-    blob->bytes.assign((uint64_t)off + 4ull * leaf_words, 0);
+    // every byte is written once (zeroing it all first took 1.4 of 7.6 ms for 300K
+    // triangles): the triangles, the sections up to the nodes (with their
+    // padding), the nodes and the leaf data
+    blob->bytes.resize((uint64_t)off + 4ull * leaf_words);
     uint8_t* b = blob->bytes.data();
+    {   // a large image's pages are first touched by the copies below: let them be large
+        // (a build of 1M triangles 46 -> 28 ms; of 300K, within the allocator's reuse, none)
+        const uintptr_t page = 1ull << 21, lo = (reinterpret_cast<uintptr_t>(b) + page - 1u) & ~(page - 1u),
+                        hi = reinterpret_cast<uintptr_t>(b + blob->bytes.size()) & ~(page - 1u);
+        if (hi > lo) madvise(reinterpret_cast<void*>(lo), hi - lo, MADV_HUGEPAGE);
+    }
+    const uint64_t tri_end = blob->ranges[TIM_RT_RANGE_TRI][0] + 12ull * n;
+    std::memset(b + tri_end, 0, blob->ranges[TIM_RT_RANGE_NODE][0] - tri_end);
     GB_CUDA(cudaMemcpyAsync(b + blob->ranges[TIM_RT_RANGE_NODE][0], d_nodes, 64ull * num_nodes, cudaMemcpyDeviceToHost,
                             st));
     GB_CUDA(cudaMemcpyAsync(b + blob->ranges[TIM_RT_RANGE_LEAF][0], d_leaf, 4ull * leaf_words, cudaMemcpyDeviceToHost,
