@@ -1142,25 +1142,57 @@ __device__ __forceinline__ void hit_normal(const SceneView& s, const uint4& rec,
     Nz = (Nn[3 * i0 + 2] * u + Nn[3 * i1 + 2] * v) + Nn[3 * i2 + 2] * w;
 }
 
+// Whether a squared distance is surely beyond a light's radius: the shader's test is
+// sqrt(d2) < radius, and the margins are above what the products and the root round by.
+__device__ __forceinline__ bool beyond(float d2, float radius) {
+    return d2 > (radius * radius) * (1.0f + 1.0f / 1048576.0f) + 1e-37f;
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The first 31 lights (a mask has no bit for more) that reach a warp's hit points, a bit
+// each: lane k measures light k from the points' box, by the operations that measure it
+// from a point, none of which can come out larger here. Called by whole warps.
+__device__ __forceinline__ uint32_t lights_in_reach(const SceneView& s, bool hit, float px, float py, float pz) {
+    const float lox = warp_min(hit ? px : INFINITY), loy = warp_min(hit ? py : INFINITY), loz = warp_min(hit ? pz : INFINITY);
+    const float hix = -warp_min(hit ? -px : INFINITY), hiy = -warp_min(hit ? -py : INFINITY), hiz = -warp_min(hit ? -pz : INFINITY);
+    const uint32_t li = threadIdx.x & 31u;
+    bool reach = false;
+    if (li < s.num_lights && li < 31u) {
+        const float* L = s.lights + 14u * li;
+        const float x = __ldg(L + 1), y = __ldg(L + 2), z = __ldg(L + 3);
+        const float ax = fmaxf(fmaxf(x - hix, lox - x), 0.0f), ay = fmaxf(fmaxf(y - hiy, loy - y), 0.0f),
+                    az = fmaxf(fmaxf(z - hiz, loz - z), 0.0f);
+        reach = __float_as_uint(__ldg(L)) == kLightSphere && !beyond(dot3(ax, ay, az, ax, ay, az), __ldg(L + 4));
+    }
+    return __ballot_sync(0xFFFFFFFFu, reach);
+}
+
 // bvhLighting.glsl:42-85 computeLighting, direct part (texColor 1): the lights whose
 // shadow-mask bit is clear (evalLighting -> evalSphereLight; an out-of-range light
 // adds nothing), then the sun (evalSunLight), summed in the shader's order.
 __device__ void direct_lit(const SceneView& s, const float* m, float px, float py, float pz, float Nx, float Ny,
-                           float Nz, float ex, float ey, float ez, uint32_t mask, const float* sun, const float* sunc,
-                           float& lx, float& ly, float& lz) {
+                           float Nz, float ex, float ey, float ez, uint32_t mask, uint32_t reach, const float* sun,
+                           const float* sunc, float& lx, float& ly, float& lz) {
     lx = 0.f; ly = 0.f; lz = 0.f;
-    for (uint32_t li = 0; li < s.num_lights && li < 31u; ++li) {
+    for (; reach; reach &= reach - 1u) {
+        const uint32_t li = (uint32_t)__ffs((int)reach) - 1u;
         if (mask & (1u << (li + 1u))) continue;
         const float* L = s.lights + 14u * li;
-        if (__float_as_uint(__ldg(L)) != kLightSphere) continue;
-        const float ax = __ldg(L + 1) - px, ay = __ldg(L + 2) - py, az = __ldg(L + 3) - pz;
-        float dd = sqrtf(dot3(ax, ay, az, ax, ay, az));
-        if (dd < __ldg(L + 4)) {
+        const float ax = __ldg(L + 1) - px, ay = __ldg(L + 2) - py, az = __ldg(L + 3) - pz, radius = __ldg(L + 4);
+        const float d2 = dot3(ax, ay, az, ax, ay, az);
+        if (beyond(d2, radius)) continue;
+        float dd = sqrtf(d2);
+        if (dd < radius) {
             const float Lx = ax / dd, Ly = ay / dd, Lz = az / dd;
             dd = fmaxf(0.01f, dd - __ldg(L + 8));
             float cx, cy, cz;
             compute_lighting(m, __ldg(L + 5), __ldg(L + 6), __ldg(L + 7), px, py, pz, Lx, Ly, Lz, Nx, Ny, Nz, ex, ey,
-                             ez, attenuation(dd, __ldg(L + 4)), cx, cy, cz);
+                             ez, attenuation(dd, radius), cx, cy, cz);
             lx = lx + cx; ly = ly + cy; lz = lz + cz;
         }
     }
@@ -1184,23 +1216,31 @@ __device__ __forceinline__ void sky_colour(float& lx, float& ly, float& lz) {
 // colour on a miss (baseRaytracingPass.glsl:81).
 __global__ void __launch_bounds__(256) k_probe_light(SceneView s, ProbeArgs d, const uint32_t* out_words, float* irr) {
     const uint32_t sample = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sample >= d.np * d.nd) return;
-    const uint32_t pl = sample / d.nd, r = sample % d.nd;
-    const uint4 rec = reinterpret_cast<const uint4*>(out_words)[2u * sample];
-    const uint32_t mask = out_words[8u * sample + 4u];
+    const bool valid = sample < d.np * d.nd;
+    uint4 rec = make_uint4(0u, 0u, 0u, __float_as_uint(kTMax));
+    float ox = 0.f, oy = 0.f, oz = 0.f, px = 0.f, py = 0.f, pz = 0.f;
+    uint32_t mask = 0u;
+    if (valid) {
+        rec = reinterpret_cast<const uint4*>(out_words)[2u * sample];
+        mask = out_words[8u * sample + 4u];
+    }
     const float t = __uint_as_float(rec.w);
+    const bool hit = t < kTMax;
+    if (hit) {
+        probe_position(d, d.p0 + sample / d.nd, ox, oy, oz);
+        const float4 dir = __ldg(d.dirs + sample % d.nd);
+        px = ox + dir.x * t; py = oy + dir.y * t; pz = oz + dir.z * t;
+    }
+    const uint32_t reach = lights_in_reach(s, hit, px, py, pz);
+    if (!valid) return;
     float lx, ly, lz;
-    if (!(t < kTMax)) {
+    if (!hit) {
         sky_colour(lx, ly, lz);
     } else {
-        float ox, oy, oz;
-        probe_position(d, d.p0 + pl, ox, oy, oz);
-        const float4 dir = __ldg(d.dirs + r);
-        const float px = ox + dir.x * t, py = oy + dir.y * t, pz = oz + dir.z * t;
         float Nx, Ny, Nz;
         hit_normal(s, rec, px, py, pz, Nx, Ny, Nz);
         const float* m = s.materials + 12u * (rec.z >> 16);
-        direct_lit(s, m, px, py, pz, Nx, Ny, Nz, ox, oy, oz, mask, d.sun, d.sunc, lx, ly, lz);
+        direct_lit(s, m, px, py, pz, Nx, Ny, Nz, ox, oy, oz, mask, reach, d.sun, d.sunc, lx, ly, lz);
     }
     irr[3u * sample] = lx;
     irr[3u * sample + 1u] = ly;
@@ -1266,24 +1306,29 @@ __global__ void __launch_bounds__(kAccumThreads) k_probe_accum(ProbeArgs d, cons
 }
 
 // ------------------------------------------------------------ camera lighting step
-__device__ __forceinline__ float mixf(float a, float b, float x) { return a * (1.0f - x) + b * x; }   // GLSL mix
-
-// fetchSH_inline.glsl:82-118 sampleSH9 with the probe mask, for one image channel:
-// v[x + 2y + 4z] are the corner values, mask bit (x + 2y + 4z) set = corner
-// masked; the shader's lerp tree, so the shader's rounding.
-__device__ __forceinline__ float masked_trilinear(const float (&v)[8], float fx, float fy, float fz, uint32_t mask) {
-    const bool m0 = !(mask & 1u), m1 = !(mask & 2u), m2 = !(mask & 4u), m3 = !(mask & 8u);
-    const bool m4 = !(mask & 16u), m5 = !(mask & 32u), m6 = !(mask & 64u), m7 = !(mask & 128u);
-    float x0 = m0 && m1 ? mixf(v[0], v[1], fx) : (m0 ? v[0] : v[1]);
-    float x1 = m2 && m3 ? mixf(v[2], v[3], fx) : (m2 ? v[2] : v[3]);
-    const bool b00 = m0 || m1, b10 = m2 || m3;
-    const float z0 = b00 && b10 ? mixf(x0, x1, fy) : (b00 ? x0 : x1);
-    x0 = m4 && m5 ? mixf(v[4], v[5], fx) : (m4 ? v[4] : v[5]);
-    x1 = m6 && m7 ? mixf(v[6], v[7], fx) : (m6 ? v[6] : v[7]);
-    const bool b01 = m4 || m5, b11 = m6 || m7;
-    const float z1 = b01 && b11 ? mixf(x0, x1, fy) : (b01 ? x0 : x1);
-    const bool bxy0 = b00 || b10, bxy1 = b01 || b11;
-    return bxy0 && bxy1 ? mixf(z0, z1, fz) : (bxy0 ? z0 : z1);
+// fetchSH_inline.glsl:82-118 sampleSH9 with the probe mask (bit x + 2y + 4z set = that
+// corner masked): GLSL mix, a * (1 - f) + b * f, of each pair along x, then y, then z; of
+// a pair with one side masked the other side as it is; of a pair with both, the second.
+// Here every pair is one product sum whatever the mask: a masked side's value is -0 and
+// its weight 0, the other's weight 1, and x * 1 + -0 * 0 is x for every x (-0 * 0 is -0,
+// the sum's neutral element); all corners masked is the shader's last corner alone. So
+// the mask costs seven pairs of weights a pixel instead of seven selects a channel, and
+// the cells' lower and upper half (corners q and q + 4) go through packed operations,
+// whose halves round as the scalar ones do. The sum is a packed FMA by a `one` that the
+// compiler can't see: it contracts a packed product and a packed add, whatever the flags.
+// (Two channels to a packed operation needs each weight twice in registers: 97 us for the
+// 1080p step of k_shade_camera's comment, against 90 us.)
+struct Lerp { float a, b; };
+__device__ __forceinline__ Lerp lerp_weights(bool has_a, bool has_b, float f) {
+    return {has_a && has_b ? 1.0f - f : (has_b && !has_a ? 0.0f : 1.0f), has_a && has_b ? f : (has_b && !has_a ? 1.0f : 0.0f)};
+}
+struct Lerp2 { uint64_t a, b; };
+__device__ __forceinline__ Lerp2 both(const Lerp& lo, const Lerp& hi) { return {pack2f(lo.a, hi.a), pack2f(lo.b, hi.b)}; }
+__device__ __forceinline__ uint64_t lerp2(uint64_t a, uint64_t b, const Lerp2& w, uint64_t one) {
+    return fma2(mul2(a, w.a), one, mul2(b, w.b));
+}
+__device__ __forceinline__ float half_of(uint32_t h, int hi) {
+    return __half2float(__ushort_as_half((unsigned short)(hi ? h >> 16 : h & 0xFFFFu)));
 }
 
 // bvhLighting.glsl:24-40 computeLPFLighting with USE_LPF_MASK: probe-grid uvw
@@ -1291,7 +1336,7 @@ __device__ __forceinline__ float masked_trilinear(const float (&v)[8], float fx,
 // (fetchSH_inline.glsl:6-31 channel layout), evalSH (lightprobHelpers.glsl:90-101)
 // and computeIndirectLighting (core/lighting.glsl:59-74, texColor 1).
 __device__ void lpf_lit(const tim_rt_pass_data& pd, const uint2* sh16, const float* m, float px, float py, float pz,
-                        float Nx, float Ny, float Nz, uint32_t mask, float& lx, float& ly, float& lz) {
+                        float Nx, float Ny, float Nz, uint32_t mask, float one, float& lx, float& ly, float& lz) {
     const uint32_t rx = pd.lpfResolution[0], ry = pd.lpfResolution[1], rz = pd.lpfResolution[2];
     const float sx = (pd.sceneMaxExtent[0] - pd.sceneMinExtent[0]) / (float)rx;
     const float sy = (pd.sceneMaxExtent[1] - pd.sceneMinExtent[1]) / (float)ry;
@@ -1306,31 +1351,45 @@ __device__ void lpf_lit(const tim_rt_pass_data& pd, const uint2* sh16, const flo
     const uint32_t ix = min((uint32_t)(int)u, rx - 2u), iy = min((uint32_t)(int)v, ry - 2u),
                    iz = min((uint32_t)(int)w, rz - 2u);
     const float fx = u - (float)(int)ix, fy = v - (float)(int)iy, fz = w - (float)(int)iz;
-    const uint64_t img = (uint64_t)rx * ry * rz;
-    float ch[7][4];
+    if ((mask & 0xFFu) == 0xFFu) mask = 0x7Fu;
+    bool on[8];
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-        float c[4][8];
+    for (int q = 0; q < 8; ++q) on[q] = !(mask & (1u << q));
+    const Lerp2 wx0 = both(lerp_weights(on[0], on[1], fx), lerp_weights(on[4], on[5], fx));
+    const Lerp2 wx1 = both(lerp_weights(on[2], on[3], fx), lerp_weights(on[6], on[7], fx));
+    const Lerp2 wy = both(lerp_weights(on[0] || on[1], on[2] || on[3], fy), lerp_weights(on[4] || on[5], on[6] || on[7], fy));
+    const Lerp wz = lerp_weights(on[0] || on[1] || on[2] || on[3], on[4] || on[5] || on[6] || on[7], fz);
+    const uint64_t img = (uint64_t)rx * ry * rz, one2 = pack2f(one, one);
+    const uint2* corner = sh16 + ((uint64_t)iz * ry + iy) * rx + ix;
+    auto sample = [&](uint32_t k, float (&ch)[4]) {
+        uint2 h[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const uint64_t texel = ((uint64_t)(iz + ((q >> 2) & 1)) * ry + (iy + ((q >> 1) & 1))) * rx + ix + (q & 1);
-            const uint2 h = __ldg(sh16 + k * img + texel);
-            c[0][q] = __half2float(__ushort_as_half((unsigned short)(h.x & 0xFFFFu)));
-            c[1][q] = __half2float(__ushort_as_half((unsigned short)(h.x >> 16)));
-            c[2][q] = __half2float(__ushort_as_half((unsigned short)(h.y & 0xFFFFu)));
-            c[3][q] = __half2float(__ushort_as_half((unsigned short)(h.y >> 16)));
+            h[q] = make_uint2(0x80008000u, 0x80008000u);   // -0
+            if (on[q]) h[q] = __ldg(corner + k * img + ((uint64_t)((q >> 2) & 1) * ry + ((q >> 1) & 1)) * rx + (q & 1));
         }
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) ch[k][cc] = masked_trilinear(c[cc], fx, fy, fz, mask);
-    }
+        for (int cc = 0; cc < 4; ++cc) {
+            uint64_t v[4];   // corner q and the one above it
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                v[q] = pack2f(half_of(cc < 2 ? h[q].x : h[q].y, cc & 1), half_of(cc < 2 ? h[q + 4].x : h[q + 4].y, cc & 1));
+            float z0, z1;
+            unpack2f(lerp2(lerp2(v[0], v[1], wx0, one2), lerp2(v[2], v[3], wx1, one2), wy, one2), z0, z1);
+            ch[cc] = z0 * wz.a + z1 * wz.b;
+        }
+    };
     const float c1 = 0.429043f, c2 = 0.511664f, c3 = 0.743125f, c4 = 0.886227f, c5 = 0.247708f;
-    float L[3];
+    float band0[4], L[3];
+    sample(0u, band0);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         // SH9Color.w[j] from the storeSH9 layout: w0 = image 0; w1..4 = images 1/3/5, w5..8 = images 2/4/6
-        const float w0 = ch[0][c], w1 = ch[1 + 2 * c][0], w2 = ch[1 + 2 * c][1], w3 = ch[1 + 2 * c][2];
-        const float w4 = ch[1 + 2 * c][3], w5 = ch[2 + 2 * c][0], w6 = ch[2 + 2 * c][1], w7 = ch[2 + 2 * c][2];
-        const float w8 = ch[2 + 2 * c][3];
+        float a[4], b[4];
+        sample(1u + 2u * c, a);
+        sample(2u + 2u * c, b);
+        const float w0 = c == 0 ? band0[0] : (c == 1 ? band0[1] : band0[2]);
+        const float w1 = a[0], w2 = a[1], w3 = a[2], w4 = a[3], w5 = b[0], w6 = b[1], w7 = b[2], w8 = b[3];
         // SH_Y00 0, Y11 1, Y10 2, Y1_1 3, Y21 4, Y2_1 5, Y2_2 6, Y20 7, Y22 8 (lightprob/lightprob.glsl)
         const float t1 = (c1 * (Nx * Nx - Ny * Ny)) * w8;
         const float t2 = ((c3 * w7) * Nz) * Nz;
@@ -1338,7 +1397,8 @@ __device__ void lpf_lit(const tim_rt_pass_data& pd, const uint2* sh16, const flo
         const float t4 = c5 * w7;
         const float t5 = (2.0f * c1) * (((w6 * Nx) * Ny + (w4 * Nx) * Nz) + (w5 * Ny) * Nz);
         const float t6 = (2.0f * c2) * ((w1 * Nx + w3 * Ny) + w2 * Nz);
-        L[c] = ((((t1 + t2) + t3) - t4) + t5) + t6;
+        const float l = ((((t1 + t2) + t3) - t4) + t5) + t6;
+        if (c == 0) L[0] = l; else if (c == 1) L[1] = l; else L[2] = l;
     }
     const uint32_t type = __float_as_uint(__ldg(m));
     const float cr = __ldg(m + 4), cg = __ldg(m + 5), cb = __ldg(m + 6);
@@ -1354,41 +1414,54 @@ __device__ void lpf_lit(const tim_rt_pass_data& pd, const uint2* sh16, const flo
 }
 
 // cameraPass.comp:78-88, the lighting step (RayTracingPass::lightingPass,
-// raytracingPass.cpp:113-135: USE_LPF, USE_LPF_MASK). One thread per output pixel
-// in row-major order (coalesced record reads and image writes); the pixel's ray is
-// the tracing step's (cameraPass.comp:46-56), output row 0 is never reached by the
-// reference's dispatch and is written as 0.
-__global__ void __launch_bounds__(256) k_shade_camera(SceneView s, tim_rt_pass_data pd, uint32_t flags,
-                                                      const uint4* tracing, const uint2* sh16, uint2* out16,
-                                                      float* out32) {
+// raytracingPass.cpp:113-135: USE_LPF, USE_LPF_MASK). One thread per output pixel, a warp
+// an 8 x 4 tile (few lights reach it, and its records, texels and image rows are whole
+// sectors); the pixel's ray is the tracing step's (cameraPass.comp:46-56), output row 0
+// is never reached by the reference's dispatch and is written as 0.
+// Bound by instruction issue (78% of the cycles; 1,200 instructions a warp, half of them
+// the probe field's 27 interpolated channels): 1920 x 1080, 16 lights, 12^3 probes took
+// 149 us (72 without the probe field) with a row of 32 pixels a warp, every light measured
+// by every pixel and the mask's selects in each channel; 90 us (41) now. Four blocks an SM
+// (64 registers, a few spilled) against three: 96 us (49); five: 105 us (38).
+__global__ void __launch_bounds__(256, 4) k_shade_camera(SceneView s, tim_rt_pass_data pd, uint32_t flags,
+                                                         const uint4* tracing, const uint2* sh16, uint2* out16,
+                                                         float* out32, float one) {
     const uint32_t W = pd.frameSize[0], H = pd.frameSize[1];
-    const uint64_t pix = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (pix >= (uint64_t)W * H) return;
-    const uint32_t px = (uint32_t)(pix % W), py = (uint32_t)(pix / W);
-    float lx = 0.f, ly = 0.f, lz = 0.f;
-    bool reached = py != 0u;
+    const uint32_t across = (W + 31u) / 32u, warp = threadIdx.x / 32u, lane = threadIdx.x & 31u;
+    const uint32_t px = blockIdx.x % across * 32u + (warp & 3u) * 8u + (lane & 7u);
+    const uint32_t py = blockIdx.x / across * 8u + (warp >> 2) * 4u + (lane >> 3);
+    const uint64_t pix = (uint64_t)py * W + px;
+    const bool valid = px < W && py < H, reached = valid && py != 0u;
+    const float ex = pd.cameraPos[0], ey = pd.cameraPos[1], ez = pd.cameraPos[2];
+    uint4 rec = make_uint4(0u, 0u, 0u, __float_as_uint(kTMax)), masks = rec;
+    float hx = 0.f, hy = 0.f, hz = 0.f;
     if (reached) {
-        const uint4 rec = __ldg(tracing + 2u * pix);
-        const uint4 masks = __ldg(tracing + 2u * pix + 1u);
-        const float t = __uint_as_float(rec.w);
-        if (!(t < kTMax)) {
-            sky_colour(lx, ly, lz);
-        } else {
-            const uint32_t ngy16 = 16u * ((H + 15u) / 16u);
-            float dx, dy, dz;
-            camera_ray(pd, px, ngy16 - py, dx, dy, dz);
-            const float ex = pd.cameraPos[0], ey = pd.cameraPos[1], ez = pd.cameraPos[2];
-            const float hx = ex + dx * t, hy = ey + dy * t, hz = ez + dz * t;
-            float Nx, Ny, Nz;
-            hit_normal(s, rec, hx, hy, hz, Nx, Ny, Nz);
-            const float* m = s.materials + 12u * (rec.z >> 16);
-            direct_lit(s, m, hx, hy, hz, Nx, Ny, Nz, ex, ey, ez, masks.x, pd.sunDir, pd.sunColor, lx, ly, lz);
-            if (!(flags & TIM_RT_SHADE_NO_LPF)) {
-                float ix, iy, iz;
-                lpf_lit(pd, sh16, m, hx, hy, hz, Nx, Ny, Nz, masks.y, ix, iy, iz);
-                lx = lx + ix; ly = ly + iy; lz = lz + iz;
-            }
+        rec = __ldg(tracing + 2u * pix);
+        masks = __ldg(tracing + 2u * pix + 1u);
+    }
+    const float t = __uint_as_float(rec.w);
+    const bool hit = t < kTMax;
+    if (hit) {
+        const uint32_t ngy16 = 16u * ((H + 15u) / 16u);
+        float dx, dy, dz;
+        camera_ray(pd, px, ngy16 - py, dx, dy, dz);
+        hx = ex + dx * t; hy = ey + dy * t; hz = ez + dz * t;
+    }
+    const uint32_t reach = lights_in_reach(s, hit, hx, hy, hz);
+    if (!valid) return;
+    float lx = 0.f, ly = 0.f, lz = 0.f;
+    if (hit) {
+        float Nx, Ny, Nz;
+        hit_normal(s, rec, hx, hy, hz, Nx, Ny, Nz);
+        const float* m = s.materials + 12u * (rec.z >> 16);
+        direct_lit(s, m, hx, hy, hz, Nx, Ny, Nz, ex, ey, ez, masks.x, reach, pd.sunDir, pd.sunColor, lx, ly, lz);
+        if (!(flags & TIM_RT_SHADE_NO_LPF)) {
+            float ix, iy, iz;
+            lpf_lit(pd, sh16, m, hx, hy, hz, Nx, Ny, Nz, masks.y, one, ix, iy, iz);
+            lx = lx + ix; ly = ly + iy; lz = lz + iz;
         }
+    } else if (reached) {
+        sky_colour(lx, ly, lz);
     }
     const uint32_t hr = __half_as_ushort(__float2half_rn(lx)), hg = __half_as_ushort(__float2half_rn(ly));
     const uint32_t hb = __half_as_ushort(__float2half_rn(lz));
@@ -1403,11 +1476,11 @@ __global__ void __launch_bounds__(256) k_shade_camera(SceneView s, tim_rt_pass_d
 
 cudaError_t launch_shade(const SceneView& s, const tim_rt_pass_data& pd, uint32_t flags, const uint32_t* tracing,
                          const uint16_t* sh16, uint16_t* out16, float* out32, cudaStream_t stream) {
-    const uint64_t npix = (uint64_t)pd.frameSize[0] * pd.frameSize[1];
-    if (npix == 0) return cudaSuccess;
-    k_shade_camera<<<(unsigned)((npix + 255u) / 256u), 256, 0, stream>>>(
+    const uint64_t blocks = ((uint64_t)pd.frameSize[0] + 31u) / 32u * (((uint64_t)pd.frameSize[1] + 7u) / 8u);
+    if (blocks == 0) return cudaSuccess;
+    k_shade_camera<<<(unsigned)blocks, 256, 0, stream>>>(
         s, pd, flags, reinterpret_cast<const uint4*>(tracing), reinterpret_cast<const uint2*>(sh16),
-        reinterpret_cast<uint2*>(out16), out32);
+        reinterpret_cast<uint2*>(out16), out32, 1.0f);
     return cudaGetLastError();
 }
 
