@@ -103,8 +103,8 @@ typedef struct {
     uint64_t primary_rays, shadow_rays, probe_rays, bounce_rays;
     float kernel_ms;          /* device time of the trace kernels (CUDA events) */
     float total_ms;           /* device time of the whole call incl. copies */
-    /* work counters, filled only with TIM_RT_TRACE_COUNT / TIM_RT_CAM_COUNT (whose
-     * binary form walks the image's own nodes): inner-node fetches (binary: 64-B node, 8-wide: 80-B node), leaf visits,
+    /* work counters, filled only with TIM_RT_TRACE_COUNT / TIM_RT_CAM_COUNT (which trace
+     * both kinds of rays in one kernel, the binary form on the image's own nodes): inner-node fetches (binary: 64-B node, 8-wide: 80-B node), leaf visits,
      * triangle tests, node-header reloads (8-wide: 32 B when a pending node is popped) */
     uint64_t node_visits, leaf_visits, tri_tests, node_reloads;
     /* camera calls: device time of the primary trace, the secondary-ray

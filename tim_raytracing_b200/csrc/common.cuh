@@ -25,6 +25,8 @@ constexpr uint32_t kFourCountShift = 27, kFourFirstMask = (1u << kFourCountShift
 constexpr uint32_t kFourBytes = 224u, kPairBytes = 112u;   // a node of the 4-wide tree, a child-pair record
 constexpr int kStackSize = 32;                  // the reference's bitstack is 32 bits wide
 
+constexpr uint32_t kQuantNodes = 0x7FFFFFu;   // 8-wide nodes a leaf reference of k_walk can name (bits 8..30)
+
 // Device view of one uploaded scene (reference layout).
 struct SceneView {
     const float4* nodes;        // PackedBVHNode: nid, n0xy, n1xy, nz (primitive_cpp.glsl:80-86)

@@ -115,25 +115,33 @@ struct SortScratch {
     size_t temp_bytes;
 };
 size_t multi_sort_temp_bytes(uint32_t total);
+// Whether a form's rays take launches of one kind each, on the tree made for that kind
+// (k_walk): in the binary form where the scene has those trees, in the 8-wide form where a
+// leaf reference can name all nodes and the stack holds the tree's levels.
+inline bool has_walk(const SceneView& v, bool wide) {
+    return wide ? v.num_wnodes && v.num_wnodes < kQuantNodes && !v.wide_root_is_leaf && v.wide_depth <= kStackSize / 2
+                : v.nodes4 != nullptr;
+}
 // What the jobs of a batch need of the kernels: the deepest tree of each kind, whether
-// every scene has the binary form's trees (SceneView::nodes4), and the kinds of rays.
+// every scene has a form's walks, and the kinds of rays.
 struct MultiNeeds {
     int depth = 1, wide_depth = 1, depth4 = 1;
-    bool four = true, any = false, closest = false;
+    bool walk[2] = {true, true};   // the binary form's, the 8-wide form's
+    bool any = false, closest = false;
     void add_scene(const SceneView& v) {
         depth = depth > (int)v.depth ? depth : (int)v.depth;
         wide_depth = wide_depth > (int)v.wide_depth ? wide_depth : (int)v.wide_depth;
         depth4 = depth4 > (int)v.depth4 ? depth4 : (int)v.depth4;
-        four = four && v.nodes4 != nullptr;
+        for (int wide = 0; wide < 2; ++wide) walk[wide] = walk[wide] && has_walk(v, wide != 0);
     }
     void add_mode(uint32_t mode) {
         any = any || mode != TIM_RT_MODE_CLOSEST;
         closest = closest || mode != TIM_RT_MODE_ANY;
     }
 };
-// Resets `counter` (two words) and launches one persistent kernel over all jobs -- in the
-// binary form, where every scene has its trees, one for the closest-hit rays and one for
-// the any-hit rays; with cfg.ray_sort != 0 the rays are first ordered by the coherence key.
+// Resets `counter` (two words) and launches one persistent kernel over the closest-hit rays
+// of all jobs and one over the any-hit rays -- or one over all, where a scene lacks the
+// form's walks; with cfg.ray_sort != 0 the rays are first ordered by the coherence key.
 cudaError_t launch_multi(const SceneView* views, const MultiJob* jobs, uint32_t njobs, uint32_t total, uint32_t* counter,
                          uint32_t* err, const MultiNeeds& needs, bool wide, const SortScratch* sort, cudaStream_t stream,
                          const LaunchConfig& cfg);

@@ -268,17 +268,20 @@ cudaError_t launch_multi(const SceneView* views, const MultiJob* jobs, uint32_t 
         perm = vb.Current();
     }
     cudaMemsetAsync(counter, 0, 8, stream);
-    if (!wide && needs.four) {
+    if (needs.walk[wide]) {
         SceneView v{};   // only the stacks' depths are taken from it
         v.depth = (uint32_t)needs.depth;
         v.depth4 = (uint32_t)needs.depth4;
+        v.wide_depth = (uint32_t)needs.wide_depth;
+        LaunchConfig c = cfg;
+        c.wide = wide;
         MultiPolicy P{views, jobs, njobs, perm, false};
         if (needs.closest) {
-            const cudaError_t e = launch_walk<false>(v, P, total, counter, err, stream, cfg, needs.any ? kPairFirst : kAlone);
+            const cudaError_t e = launch_rays<false>(v, P, total, counter, err, stream, c, needs.any ? kPairFirst : kAlone);
             if (e != cudaSuccess || !needs.any) return e;
         }
         P.any = true;
-        return launch_walk<true>(v, P, total, counter + 1, err, stream, cfg, needs.closest ? kPairSecond : kAlone);
+        return launch_rays<true>(v, P, total, counter + 1, err, stream, c, needs.closest ? kPairSecond : kAlone);
     }
     switch (cfg.block) {
         case 64:

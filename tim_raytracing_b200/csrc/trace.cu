@@ -784,9 +784,16 @@ static cudaError_t launch_persistent(const SceneView& s, const Policy& P, uint32
     return cudaGetLastError();
 }
 
-// Launches of the binary form take the two trees where the scene has them; the
-// counting kernels count the plain binary walk's work.
-static bool use_four(const SceneView& s, const LaunchConfig& cfg) { return !cfg.wide && s.nodes4 && !cfg.stats; }
+static bool use_walk(const SceneView& s, const LaunchConfig& cfg) { return !cfg.stats && has_walk(s, cfg.wide); }
+
+// The general kernel: counting launches, two-level scenes, scenes without the trees of the
+// walks.
+template <class Policy>
+static cudaError_t launch_general(const SceneView& s, const Policy& P, uint32_t n, uint32_t* counter, uint32_t* err,
+                                  cudaStream_t stream, const LaunchConfig& cfg) {
+    return cfg.wide ? launch_persistent<true>(s, P, n, counter, err, stream, cfg)
+                    : launch_persistent<false>(s, P, n, counter, err, stream, cfg);
+}
 
 cudaError_t launch_trace_batch(const SceneView& s, const tim_rt_ray* rays, uint32_t n, uint32_t mode, uint32_t* hit,
                                uint32_t* nid, float* bary, uint32_t* counter, uint32_t* err, cudaStream_t stream,
@@ -797,17 +804,16 @@ cudaError_t launch_trace_batch(const SceneView& s, const tim_rt_ray* rays, uint3
         static_cast<BatchPolicy&>(T) = P;
         return launch_persistent<false>(s, T, n, counter, err, stream, cfg);
     }
-    if (cfg.wide) return launch_persistent<true>(s, P, n, counter, err, stream, cfg);
-    if (!use_four(s, cfg)) return launch_persistent<false>(s, P, n, counter, err, stream, cfg);
-    if (P.mode == TIM_RT_MODE_CLOSEST) return launch_walk<false>(s, P, n, counter, err, stream, cfg);
-    if (P.mode == TIM_RT_MODE_ANY) return launch_walk<true>(s, P, n, counter, err, stream, cfg);
+    if (!use_walk(s, cfg)) return launch_general(s, P, n, counter, err, stream, cfg);
+    if (P.mode == TIM_RT_MODE_CLOSEST) return launch_rays<false>(s, P, n, counter, err, stream, cfg);
+    if (P.mode == TIM_RT_MODE_ANY) return launch_rays<true>(s, P, n, counter, err, stream, cfg);
     KindBatchPolicy K;
     static_cast<BatchPolicy&>(K) = P;
     K.kind = 0u;
-    const cudaError_t e = launch_walk<false>(s, K, n, counter, err, stream, cfg, kPairFirst);
+    const cudaError_t e = launch_rays<false>(s, K, n, counter, err, stream, cfg, kPairFirst);
     if (e != cudaSuccess) return e;
     K.kind = TIM_RT_RAY_ANY;
-    return launch_walk<true>(s, K, n, counter + 1, err, stream, cfg, kPairSecond);
+    return launch_rays<true>(s, K, n, counter + 1, err, stream, cfg, kPairSecond);
 }
 
 // The queue's counters (laid out as kernels.h says) as a generator and its launch use them.
@@ -841,20 +847,19 @@ static cudaError_t launch_secondary(const SceneView& s, const GenParams& g, uint
     P.closest_last = g.closest_last;
     P.seg0 = 0u;
     P.seg1 = nb * kNumKinds;
-    if (cfg.wide) return launch_persistent<true>(s, P, 0u, counters + 1, err, stream, cfg);
-    if (!g.closest_last) return launch_persistent<false>(s, P, 0u, counters + 1, err, stream, cfg);
+    if (!g.closest_last) return launch_general(s, P, 0u, counters + 1, err, stream, cfg);
     if (bounces) {
         P.seg0 = nb * kKindBounce;
         // with bands both launches must get on together, as a band is final after both:
         // half of the GPU for the bounce rays (the 1080p frame through host buffers takes
         // 2.57 ms with a half, 2.58 with a third, 2.62 with a quarter)
-        const cudaError_t e = launch_walk<false>(s, P, 0u, counters + 3u + 54u * nb, err, stream, cfg, kPairFirst,
+        const cudaError_t e = launch_rays<false>(s, P, 0u, counters + 3u + 54u * nb, err, stream, cfg, kPairFirst,
                                                  nb > 1u ? 2 : 1);
         if (e != cudaSuccess) return e;
         P.seg0 = 0u;
     }
     P.seg1 = nb * kKindBounce;
-    return launch_walk<true>(s, P, 0u, counters + 1, err, stream, cfg, bounces ? kPairSecond : kAlone);
+    return launch_rays<true>(s, P, 0u, counters + 1, err, stream, cfg, bounces ? kPairSecond : kAlone);
 }
 
 uint32_t camera_queue_segment(uint32_t W, uint32_t H) { return W * H; }
@@ -904,9 +909,8 @@ cudaError_t launch_camera(const SceneView& s, const tim_rt_pass_data& pd, uint32
     LaunchConfig pcfg = cfg;
     pcfg.refill_min = 32;
     if (flags & TIM_RT_CAM_PRIMARY_BINARY) pcfg.wide = false;
-    cudaError_t e = pcfg.wide ? launch_persistent<true>(s, CP, items, counters + 0, err, stream, pcfg)
-                    : use_four(s, pcfg) ? launch_walk<false>(s, CP, items, counters + 0, err, stream, pcfg)
-                                        : launch_persistent<false>(s, CP, items, counters + 0, err, stream, pcfg);
+    cudaError_t e = use_walk(s, pcfg) ? launch_rays<false>(s, CP, items, counters + 0, err, stream, pcfg)
+                                      : launch_general(s, CP, items, counters + 0, err, stream, pcfg);
     if (e != cudaSuccess) return e;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[1], stream);
     GenParams g;
@@ -924,7 +928,7 @@ cudaError_t launch_camera(const SceneView& s, const tim_rt_pass_data& pd, uint32
     g.q_pixel = q_pixel;
     g.item0 = item0;
     g.item1 = item1;
-    queue_counters(counters, qb, flags_host, use_four(s, cfg), g);
+    queue_counters(counters, qb, flags_host, use_walk(s, cfg), g);
     k_gen_secondary<<<(items + 255u) / 256u, 256, 0, stream>>>(s, g);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[2], stream);
@@ -1492,9 +1496,8 @@ cudaError_t launch_probes(const SceneView& s, const ProbeArgs& d, uint32_t* out,
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[0], stream);
     LaunchConfig pcfg = cfg;
     pcfg.wide = cfg.wide && !cfg.primary_binary;
-    cudaError_t e = pcfg.wide ? launch_persistent<true>(s, PP, n, counters + 0, err, stream, pcfg)
-                    : use_four(s, pcfg) ? launch_walk<false>(s, PP, n, counters + 0, err, stream, pcfg)
-                                        : launch_persistent<false>(s, PP, n, counters + 0, err, stream, pcfg);
+    cudaError_t e = use_walk(s, pcfg) ? launch_rays<false>(s, PP, n, counters + 0, err, stream, pcfg)
+                                      : launch_general(s, PP, n, counters + 0, err, stream, pcfg);
     if (e != cudaSuccess) return e;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[1], stream);
     GenParams g{};
@@ -1504,7 +1507,7 @@ cudaError_t launch_probes(const SceneView& s, const ProbeArgs& d, uint32_t* out,
     QueueBands qb{};
     qb.n = 1;
     qb.cap[0] = n;
-    queue_counters(counters, qb, nullptr, use_four(s, cfg), g);
+    queue_counters(counters, qb, nullptr, use_walk(s, cfg), g);
     k_probe_gen<<<(n + 255u) / 256u, 256, 0, stream>>>(s, d, g, leaf_nid);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[2], stream);

@@ -62,6 +62,10 @@
 // near-tie, a hit grazing its leaf box: about one ray in 10^5) is traced again
 // from the root by the binary walk (binary_walk below), which reproduces the
 // reference's order exactly.
+//
+// Launches whose scene has_walk (kernels.h) trace each kind of ray by a kernel of its own
+// (trace_quant.cuh); the walk here is that of counting launches, single-leaf scenes and
+// trees too large for it.
 #pragma once
 #include "common.cuh"
 #include "trace_plain.cuh"

@@ -1,10 +1,11 @@
-// walk.cuh -- the persistent kernel of the binary form's rays (k_walk) and its launcher,
-// for the single-scene launches (trace.cu) and the batched ones (multi.cu).
+// walk.cuh -- the persistent kernel for rays of one kind (k_walk) and its launcher, for the
+// single-scene launches (trace.cu) and the batched ones (multi.cu).
 #pragma once
 #include "common.cuh"
 #include "kernels.h"
 #include "trace_any.cuh"
 #include "trace_pair.cuh"
+#include "trace_quant.cuh"
 
 namespace timrt {
 
@@ -75,9 +76,10 @@ __device__ __forceinline__ void refill_filtered(const Policy& P, uint32_t n, uin
 }
 
 // Shared-memory words a thread of k_walk has beside its stack: the ray's origin and
-// direction, in batched launches what names its job and scene, and two of its warp's.
-template <class Policy>
-constexpr int walk_words = many_scenes<Policy>::value ? 11 : 8;
+// direction, in batched launches what names its job and scene, in the 8-wide form its
+// tmax, and two of its warp's.
+template <class Policy, bool QUANT>
+constexpr int walk_words = (many_scenes<Policy>::value ? 11 : 8) + (QUANT ? 1 : 0);
 // A warp's leaves are spread over its lanes up to this many triangles (two rounds; a leaf
 // of four on each lane's own takes four). 1M mixed rays / the 16-scene batch / probe rays:
 // 0.463 / 2.11 / 1.00 ms with 32, 0.453 / 2.01 / 0.97 with 64, 0.453 / 1.98 / 0.96 with
@@ -86,24 +88,26 @@ constexpr uint32_t kSpreadMost = 64u;
 // Threads per SM the registers are cut to. The batches' kernels hold more per ray and
 // their rays miss the L1 most: 3 blocks without spills instead of 4 with (1M mixed rays
 // 0.427 against 0.451 ms, the 16-scene batch 2.26 against 2.36); the others 4 blocks
-// (camera rays 0.33 against 0.36 ms, probe rays 1.02 against 1.09).
-template <class Policy>
-constexpr int walk_threads = filters<Policy>::value ? 768 : 1024;
+// (camera rays 0.33 against 0.36 ms, probe rays 1.02 against 1.09). In the 8-wide form
+// the closest-hit rays take 3 (secondary rays of a frame 1.42 -> 1.39 ms).
+template <class Policy, bool ANY, bool QUANT>
+constexpr int walk_threads = filters<Policy>::value || (QUANT && !ANY) ? 768 : 1024;
 
-// Rays of one kind on their own tree: any-hit rays on the 4-wide one (trace_any.cuh),
-// closest-hit rays on the binary one's child pairs (trace_pair.cuh). The same
+// Rays of one kind on their own tree: in the binary form any-hit rays on the 4-wide one
+// (trace_any.cuh), closest-hit rays on the binary one's child pairs (trace_pair.cuh); in
+// the 8-wide form (QUANT) both on the quantised one (trace_quant.cuh). The same
 // persistent loop, with the ray's place in st.node alone -- an inner node, a leaf, or
 // kAnyIdle, which is also the lowest word of its stack, so that popping it ends the
 // walk. sdepth: stack words per thread; an any-hit ray that would need more takes the
-// plain binary walk, a closest-hit ray never does.
+// plain binary walk, no other ray ever does.
 //
 // A batch of both kinds is two launches (kPairFirst, kPairSecond) that may overlap: the
 // first lets the second start as soon as its own blocks leave room, so that the second's
 // rays fill the first's tail; neither reads what the other writes, and the second ends
 // only after the first has.
 constexpr int kAlone = 0, kPairFirst = 1, kPairSecond = 2;
-template <int BLOCK, bool ANY, class Policy>
-__global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(SceneView s, Policy P, uint32_t n_static, uint32_t* counter,
+template <int BLOCK, bool ANY, bool QUANT, class Policy>
+__global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOCK) k_walk(SceneView s, Policy P, uint32_t n_static, uint32_t* counter,
                                                               uint32_t* err, int sdepth, int knobs) {
     extern __shared__ uint32_t stack_mem[];
     // knobs: refill threshold (bits 0..7), phase-switch threshold (bits 8..15), role in a pair (bits 16..)
@@ -116,9 +120,10 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
     uint32_t* org = stk + (size_t)sdepth * BLOCK;   // the ray's origin and direction
     uint32_t* dir = org + 3 * BLOCK;
     uint32_t* own = dir + 3 * BLOCK;                 // many_scenes<Policy>: the ray's job, its place there, its scene
-    uint32_t* tab = stack_mem + (size_t)(sdepth + walk_words<Policy> - 2) * BLOCK + (threadIdx.x & ~31u);   // of the warp
+    uint32_t* tab = stack_mem + (size_t)(sdepth + walk_words<Policy, QUANT> - 2) * BLOCK + (threadIdx.x & ~31u);   // of the warp
     uint32_t* res = tab + BLOCK;
-    uint32_t* pool = stack_mem + (size_t)(sdepth + walk_words<Policy>) * BLOCK + (threadIdx.x & ~31u);   // filters<Policy> only
+    uint32_t* far = own + (many_scenes<Policy>::value ? 3 * BLOCK : 0);   // QUANT: the ray's tmax
+    uint32_t* pool = stack_mem + (size_t)(sdepth + walk_words<Policy, QUANT>) * BLOCK + (threadIdx.x & ~31u);   // filters<Policy> only
     uint32_t used = 0, have = 0;
     // Where few lanes hold leaves at a time -- closest-hit rays (9 to 14 of 32), batches in
     // any order (5) -- their triangles are spread over the warp. The any-hit rays of frames
@@ -144,7 +149,11 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
                 own[BLOCK] = st.slot2;
                 own[2 * BLOCK] = st.view;
             }
-            if (ANY) any_init(scene(), st, bottom);
+            if constexpr (QUANT) {
+                *far = __float_as_uint(st.t);
+                quant_init<ANY>(st, bottom);
+                st.refs = reinterpret_cast<const char*>(scene().wnodes);
+            } else if (ANY) any_init(scene(), st, bottom);
             else pair_init(scene(), st, bottom);
             put3<BLOCK>(org, st.r.ox, st.r.oy, st.r.oz);
             put3<BLOCK>(dir, st.r.dx, st.r.dy, st.r.dz);
@@ -166,7 +175,10 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
                 }
                 if (ANY) get3<BLOCK>(org, st.r.ox, st.r.oy, st.r.oz);
                 get3<BLOCK>(dir, st.r.dx, st.r.dy, st.r.dz);
-                if (ANY) any_finish_or_walk(scene(), st, err);
+                if constexpr (QUANT) {
+                    st.t0 = __uint_as_float(*far);
+                    quant_finish<ANY>(scene(), st, P.wants_bary(st), err);
+                } else if (ANY) any_finish_or_walk(scene(), st, err);
                 else pair_finish(scene(), st, P.wants_nid(st), P.wants_bary(st));
                 P.store(s, idx, st, st.t);   // an any-hit ray's t stays its tmax
             }
@@ -196,8 +208,12 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
                 if (leaves && 32u * visiting <= phase_sw * (visiting + leaves)) break;
             }
             if ((int)st.node >= 0) {
-                const char* refs = many_scenes<Policy>::value ? st.refs : ANY ? four_refs(s) : pair_refs(s);
-                if (ANY) any_advance<BLOCK>(st, refs, limit);
+                const char* refs = many_scenes<Policy>::value ? st.refs
+                                   : QUANT                    ? reinterpret_cast<const char*>(s.wnodes)
+                                   : ANY                      ? four_refs(s)
+                                                              : pair_refs(s);
+                if (QUANT) quant_advance<BLOCK, ANY>(st, refs, bottom);
+                else if (ANY) any_advance<BLOCK>(st, refs, limit);
                 else pair_advance<BLOCK>(st, refs, dir);
             }
         }
@@ -205,7 +221,7 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
         // one, spread over all lanes
         const bool leaf = (int)st.node < 0 && st.node != kAnyIdle;
         uint32_t first = 0, cnt = 0;
-        if (leaf) cnt = leaf_ref(scene(), st.node, first);
+        if (leaf) cnt = QUANT ? quant_leaf(scene(), st.node, first) : leaf_ref(scene(), st.node, first);
         uint32_t incl = cnt, total = 0xFFFFFFFFu;
         if constexpr (kSpread) {
 #pragma unroll
@@ -221,7 +237,8 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
                 Ray r{st.r.ox, st.r.oy, st.r.oz, 0.f, 0.f, 0.f};
                 if (ANY) get3<BLOCK>(org, r.ox, r.oy, r.oz);
                 get3<BLOCK>(dir, r.dx, r.dy, r.dz);
-                over = leaf_triangles<ANY>(scene().ptris, st, r, first, cnt);
+                over = QUANT ? quant_triangles<ANY>(scene().wtris, st, r, first, cnt, !P.wants_nid(st))
+                             : leaf_triangles<ANY>(scene().ptris, st, r, first, cnt);
             }
         } else if (kSpread && total) {
             const uint32_t excl = incl - cnt, owners = __ballot_sync(0xFFFFFFFFu, cnt != 0u);
@@ -241,8 +258,11 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
                     Ray r;
                     get3<BLOCK>(org + (int)shift, r.ox, r.oy, r.oz);
                     get3<BLOCK>(dir + (int)shift, r.dx, r.dy, r.dz);
-                    const float4* tp = s.ptris;
-                    if constexpr (many_scenes<Policy>::value) tp = P.views[own[2 * BLOCK + (int)shift]].ptris;
+                    const float4* tp = QUANT ? s.wtris : s.ptris;
+                    if constexpr (many_scenes<Policy>::value) {
+                        const SceneView& view = P.views[own[2 * BLOCK + (int)shift]];
+                        tp = QUANT ? view.wtris : view.ptris;
+                    }
                     tp += 3ull * tri;
                     const float4 A = __ldg(tp), B = __ldg(tp + 1), C = __ldg(tp + 2);
                     float u, v;
@@ -266,7 +286,9 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
                         for (; m; m &= m - 1u) {
                             const uint32_t k = (uint32_t)__ffs(m) - 1u;
                             const float tk = __uint_as_float(res[k]);
-                            if (tk < st.t) {   // the rule triangle by triangle, as leaf_triangles has it
+                            if constexpr (QUANT) {
+                                if (tk < st.t) quant_hit(scene().wtris, st, first - excl + b + k, tk, !P.wants_nid(st));
+                            } else if (tk < st.t) {   // the rule triangle by triangle, as leaf_triangles has it
                                 st.t = tk - kOffsetRayCollision;
                                 st.nid = first - excl + b + k;
                                 st.hit = true;
@@ -282,6 +304,10 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy> / BLOCK) k_walk(Sc
             if (ANY && over) {
                 st.hit = true;
                 st.node = kAnyIdle;
+            } else if constexpr (QUANT) {
+                const uint32_t rest = st.node & (st.node - 1u);
+                if (rest & 0xFFu) st.node = rest;
+                else quant_next<BLOCK, ANY>(st, bottom);
             } else {
                 st.node = stack_pop<BLOCK>(st.top);
             }
@@ -314,12 +340,12 @@ static int grid_of(GridCache& cache, K* kernel, int depth, int max_depth) {
 // against 2.01 ms (16 overflow often enough there for the binary walk to show).
 constexpr int kAnyStack = 24, kWalkStack = kStackSize + 2;
 
-template <int BLOCK, bool ANY, class Policy>
+template <int BLOCK, bool ANY, bool QUANT, class Policy>
 static cudaError_t launch_walk_block(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter,
                                      uint32_t* err, int depth, int knobs, int role, int share, cudaStream_t stream) {
     static GridCache cache;
-    const int words = depth + walk_words<Policy>;
-    const int grid = grid_of<BLOCK, Policy>(cache, k_walk<BLOCK, ANY, Policy>, words, kWalkStack + walk_words<Policy>);
+    const int words = depth + walk_words<Policy, QUANT>;
+    const int grid = grid_of<BLOCK, Policy>(cache, k_walk<BLOCK, ANY, QUANT, Policy>, words, kWalkStack + walk_words<Policy, QUANT>);
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(share > 1 && grid >= share ? grid / share : grid);
     lc.blockDim = dim3(BLOCK);
@@ -332,32 +358,43 @@ static cudaError_t launch_walk_block(const SceneView& s, const Policy& P, uint32
         lc.attrs = &at;
         lc.numAttrs = 1;
     }
-    return cudaLaunchKernelEx(&lc, k_walk<BLOCK, ANY, Policy>, s, P, n_static, counter, err, depth, knobs | role << 16);
+    return cudaLaunchKernelEx(&lc, k_walk<BLOCK, ANY, QUANT, Policy>, s, P, n_static, counter, err, depth, knobs | role << 16);
 }
 
 // One launch of k_walk, or one of a pair (of which the first may be given a share of the
 // GPU only). Stack words: a closest-hit ray leaves one child a level waiting, an any-hit
-// ray up to three slots, of which kAnyStack words are kept; the end marker; and the word
-// above the top, which a push writes whether it keeps it or not.
-template <bool ANY, class Policy>
+// ray up to three slots, of which kAnyStack words are kept, a ray of the 8-wide form two
+// words a level; the end marker; and the word above the top, which a push writes whether
+// it keeps it or not.
+template <bool ANY, bool QUANT = false, class Policy>
 static cudaError_t launch_walk(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter, uint32_t* err,
                                cudaStream_t stream, const LaunchConfig& cfg, int role = kAlone, int share = 1) {
     int depth = (int)s.depth + 2;
     LaunchConfig c = cfg;
-    if (ANY) {
+    if (QUANT) {
+        depth = 2 * (int)s.wide_depth + 2;
+    } else if (ANY) {
         depth = 3 * (int)s.depth4 + 2;
         depth = depth < 6 ? 6 : (depth > kAnyStack ? kAnyStack : depth);
-        // any-hit rays of one origin's neighbourhood profit more from starting together (they
-        // read the same nodes; the L1 binds this walk): 16 -> 24 idle lanes, 0.81 -> 0.73 ms
-        // for the 5.1M any-hit rays of the 1080p frame. launch_knobs limits it to 32.
-        c.refill_min = cfg.refill_min + cfg.refill_min / 2;
     }
+    // any-hit rays of one origin's neighbourhood profit more from starting together (they
+    // read the same nodes; the L1 binds this walk): 16 -> 24 idle lanes, 0.81 -> 0.73 ms
+    // for the 5.1M any-hit rays of the 1080p frame. launch_knobs limits it to 32.
+    if (ANY) c.refill_min = cfg.refill_min + cfg.refill_min / 2;
     const int knobs = launch_knobs(c);
     switch (cfg.block) {
-        case 64: return launch_walk_block<64, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
-        case 256: return launch_walk_block<256, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
-        default: return launch_walk_block<128, ANY>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
+        case 64: return launch_walk_block<64, ANY, QUANT>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
+        case 256: return launch_walk_block<256, ANY, QUANT>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
+        default: return launch_walk_block<128, ANY, QUANT>(s, P, n_static, counter, err, depth, knobs, role, share, stream);
     }
+}
+
+// launch_walk for the form cfg asks for (has_walk).
+template <bool ANY, class Policy>
+static cudaError_t launch_rays(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter, uint32_t* err,
+                               cudaStream_t stream, const LaunchConfig& cfg, int role = kAlone, int share = 1) {
+    return cfg.wide ? launch_walk<ANY, true>(s, P, n_static, counter, err, stream, cfg, role, share)
+                    : launch_walk<ANY, false>(s, P, n_static, counter, err, stream, cfg, role, share);
 }
 
 }  // namespace timrt
