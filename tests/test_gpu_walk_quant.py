@@ -43,6 +43,27 @@ def test_batch_sizes(ctx, native, oracle_mod, n):
         ctx.free_scene(sid)
 
 
+@pytest.mark.parametrize("n", [147, 1777, 5000, 14209, 37888, 37889])
+def test_few_rays(ctx, native, oracle_mod, n):
+    """Ray counts that are spread over the warps, one to eight to each, and just above, in
+    both forms."""
+    from tim_raytracing_b200 import scenes
+    s = scenes.heightfield_scene(seed=23, grid=24, n_spheres=4)
+    img = native.build_bvh(s)
+    sid = ctx.upload(img, s, quant8=True)
+    try:
+        sc, rays = oracle_mod.Scene(img, s.positions, s.normals), _rays(np.random.default_rng(n), n, (0, 0, 0), (20, 20, 6))
+        _check(native, oracle_mod, ctx, sid, sc, rays)
+        for mode in (native.MODE_CLOSEST, native.MODE_ANY, native.MODE_PER_RAY):
+            hit, nid, bary, _ = ctx.trace(sid, rays, mode)
+            oh, on, ob, _ = oracle_mod.trace(sc, rays, mode)
+            assert np.array_equal(hit.view(np.uint32), oh.view(np.uint32)), mode
+            assert np.array_equal(nid, on), mode
+            assert np.array_equal(bary.view(np.uint32), ob.view(np.uint32)), mode
+    finally:
+        ctx.free_scene(sid)
+
+
 @pytest.mark.parametrize("tris,leaf", [(1, 4), (2, 1), (3, 1), (9, 1), (40, 1), (3000, 15), (3000, 60)])
 def test_leaf_sizes_and_small_trees(ctx, native, oracle_mod, tris, leaf):
     from tim_raytracing_b200 import scenes

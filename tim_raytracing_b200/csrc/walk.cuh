@@ -40,25 +40,25 @@ __device__ __forceinline__ uint32_t items_of(const Policy& P, uint32_t n) {
 }
 
 // Hands the items of a batch that a filtering policy (filters<Policy>) keeps to the
-// idle lanes of a warp: 32 items at a time are looked at, those kept wait in `pool`
+// idle lanes of a warp: `batch` items (up to 32) at a time are looked at, those kept wait in `pool`
 // (32 words of shared memory a warp) until lanes take them. start(item) is called by
 // the lanes that got one; sets exhausted once the batch is used up.
 template <class Policy, class Start>
 __device__ __forceinline__ void refill_filtered(const Policy& P, uint32_t n, uint32_t* counter, uint32_t* pool,
-                                                uint32_t need, uint32_t& used, uint32_t& have, bool& exhausted,
-                                                Start start) {
+                                                uint32_t need, uint32_t batch, uint32_t& used, uint32_t& have,
+                                                bool& exhausted, Start start) {
     const uint32_t lane = threadIdx.x & 31u;
     while (need) {
         if (used == have) {
             uint32_t base = 0;
-            if (lane == 0u) base = atomicAdd(counter, 32u);
+            if (lane == 0u) base = atomicAdd(counter, batch);
             base = __shfl_sync(0xFFFFFFFFu, base, 0);
             if (base >= n) {
                 exhausted = true;
                 return;
             }
             const uint32_t item = base + lane;
-            const bool mine = item < n && P.keeps(item);
+            const bool mine = lane < batch && item < n && P.keeps(item);
             const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine);
             if (mine) pool[__popc(m & lanemask_lt())] = item;
             __syncwarp();
@@ -85,6 +85,11 @@ constexpr int walk_words = (many_scenes<Policy>::value ? 11 : 8) + (QUANT ? 1 : 
 // 0.463 / 2.11 / 1.00 ms with 32, 0.453 / 2.01 / 0.97 with 64, 0.453 / 1.98 / 0.96 with
 // 96, which costs the bounce and camera rays 2 %.
 constexpr uint32_t kSpreadMost = 64u;
+// A ray alone on its warp waits for no other's loads and leaves: launches of few rays are
+// bound by that latency, not by the GPU's width. Closest-hit rays in the 100K-triangle
+// scene, 32 rays a warp / spread: 100 rays 64 / 44 us, 1,000 87 / 64, 4,000 106 / 92,
+// 16,000 140 / 134; any-hit 53 / 42, 66 / 49, 77 / 70, 100 / 98; 64,000 (14 lanes) no less.
+constexpr uint32_t kFewLanes = 8u;
 // Threads per SM the registers are cut to. The batches' kernels hold more per ray and
 // their rays miss the L1 most: 3 blocks without spills instead of 4 with (1M mixed rays
 // 0.427 against 0.451 ms, the 16-scene batch 2.26 against 2.36); the others 4 blocks
@@ -112,11 +117,18 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOC
     extern __shared__ uint32_t stack_mem[];
     // knobs: refill threshold (bits 0..7), phase-switch threshold (bits 8..15), role in a pair (bits 16..)
     if ((knobs >> 16) == kPairFirst) cudaTriggerProgrammaticLaunchCompletion();
-    const int refill_min = knobs & 0xFF;
     const uint32_t phase_sw = (uint32_t)(knobs >> 8) & 0xFFu;
     uint32_t* stk = stack_mem + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n = items_of(P, n_static);
+    // Few rays are spread over all warps, up to kFewLanes lanes of each taking part (the
+    // rest help with leaf triangles); one launch of a pair takes half of the blocks, which
+    // leaves room for the other's rays.
+    const uint32_t blocks = (knobs >> 16) == kAlone ? gridDim.x : (gridDim.x + 1u) / 2u, warps = blocks * (BLOCK / 32);
+    const bool few = n <= kFewLanes * warps;
+    const uint32_t lanes = few ? max(1u, (n + warps - 1u) / warps) : 32u;
+    const uint32_t all = lanes == 32u ? 0xFFFFFFFFu : (1u << lanes) - 1u;
+    const int refill_min = min(knobs & 0xFF, (int)lanes);
     uint32_t* org = stk + (size_t)sdepth * BLOCK;   // the ray's origin and direction
     uint32_t* dir = org + 3 * BLOCK;
     uint32_t* own = dir + 3 * BLOCK;                 // many_scenes<Policy>: the ray's job, its place there, its scene
@@ -134,7 +146,7 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOC
 
     TravState st;
     st.node = kAnyIdle;
-    bool pending = false, exhausted = false;
+    bool pending = false, exhausted = few && blockIdx.x >= blocks;
     uint32_t idx = 0;
     stk[0] = kAnyIdle;
     auto scene = [&]() -> const SceneView& {
@@ -163,8 +175,8 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOC
         }
     };
     for (;;) {
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, st.node == kAnyIdle);
-        if (idle && (exhausted || __popc(idle) >= refill_min || idle == 0xFFFFFFFFu)) {
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, st.node == kAnyIdle) & all;
+        if (idle && (exhausted || __popc(idle) >= refill_min || idle == all)) {
             const bool stored = pending && st.node == kAnyIdle;
             if (stored) {
                 pending = false;
@@ -184,9 +196,9 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOC
             }
             if constexpr (finishes<Policy>::value) P.finished(stored, st.slot2);
             if (exhausted) {
-                if (idle == 0xFFFFFFFFu) break;
+                if (idle == all) break;
             } else if constexpr (filters<Policy>::value) {
-                refill_filtered(P, n, counter, pool, idle, used, have, exhausted, start);
+                refill_filtered(P, n, counter, pool, idle, lanes, used, have, exhausted, start);
             } else {
                 const int leader = __ffs(idle) - 1;
                 uint32_t base = 0;
