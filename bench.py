@@ -173,8 +173,12 @@ def plain_bytes(st, prefix=""):
     return 64 * g("node_visits") + 16 * g("leaf_visits") + 48 * g("tri_tests")
 
 
-BYTES_WIDE = "80 per 8-wide node + 32 per node-header reload + 48 per triangle test (device counts)"
-BYTES_PLAIN = "64 per node + 16 per leaf record + 48 per triangle test (device counts)"
+# of the counting kernels' walks: the timed kernels answer the same rays from the trees made
+# for each kind of ray (4-wide nodes and child pairs; the 8-wide nodes without header reloads)
+BYTES_WIDE = ("80 per 8-wide node + 32 per node-header reload + 48 per triangle test (device counts of the "
+              "8-wide walk by the counting kernel)")
+BYTES_PLAIN = ("64 per node + 16 per leaf record + 48 per triangle test (device counts of the reference's binary "
+               "walk by the counting kernel)")
 
 
 # ---------------------------------------------------------------- the oracle: checker and CPU baseline only
@@ -285,7 +289,7 @@ def parity_room(room, threads):
 
 def parity_batched(jobs, threads):
     """Config 3: every ray of every job (20.9M rays, 64 scenes) traced by the
-    oracle and compared with both forms' k_multi records."""
+    oracle and compared with both forms' records."""
     from oracle import oracle as O
     from tim_raytracing_b200 import _native as N
     diff = {"plain": 0, "wide": 0}
@@ -530,7 +534,8 @@ def bench_batched(N, ctx, dev, steps, warmup, l2_gbs, keep_for_parity):
                      "separate_launches_ms": float(np.median(sep)),
                      "separate_launches_value": total / (float(np.median(sep)) / 1e3) / 1e6,
                      "roofline": roofline(abytes, med, l2_gbs, f"k_multi_{form}",
-                                          f"k_multi<{tune['block']}, {1 if form == 'wide' else 0}> (64 scenes)",
+                                          f"k_walk<{tune['block']}, 0 | 1, {1 if form == 'wide' else 0}, MultiPolicy> (64 scenes: the closest-hit "
+                                          "and the any-hit launch, overlapped)",
                                           BYTES_WIDE if form == "wide" else BYTES_PLAIN)}
     ctx.set_launch_config()
     differing = 0
@@ -627,7 +632,7 @@ def bench_probes(N, ctx, l2_gbs, keep_for_parity, reps=5):
         _, _, _, stc = ctx.trace(sid, rays, N.MODE_CLOSEST | N.TRACE_COUNT, want_nid=False, want_bary=False)
         out[set_name]["roofline_probe_rays"] = roofline(
             plain_bytes(stc), out[set_name]["plain_binary"]["probe_ray_launch_ms"], l2_gbs, key,
-            "k_persistent<256, 0, 0, ProbePolicy> (probe rays, binary walk)", BYTES_PLAIN)
+            "k_walk<256, 0, 0, ProbePolicy> (probe rays, binary walk)", BYTES_PLAIN)
         del rays
     dirs = sets["octahedral"][0]
     # FP16 texel storage error against FP64 averaging of the same radiance
@@ -814,7 +819,7 @@ def bench_jobs_100k(N, ctx, dev, frame_scene, sid, steps=10):
     generator), traced (a) in the plain form as one binary-BVH launch per job, the
     way a caller without batching dispatches them (each launch then lasts at least
     one ray's chain of dependent node loads), and (b) in the quantised batched form
-    as one 8-wide k_multi launch over all jobs in a CUDA graph; also the two mixed
+    as one 8-wide batch over all jobs in a CUDA graph; also the two mixed
     cases. Device-resident rays; hit records must be identical. Most of the gain
     of (b) over (a) is the batching, not the quantisation: the plain batched form
     is reported beside it."""
@@ -1001,11 +1006,11 @@ def main():
     ap.add_argument("--profile", choices=["plain", "wide", "pipelined", "batched-plain", "batched-wide",
                                           "probes-plain", "probes-wide", "probes-stratified", "shade", "build"],
                     help="only run a small, fixed launch sequence for ncu and exit: plain / wide = two frames of "
-                         "one form (per frame one primary and one secondary k_persistent launch); pipelined = two "
+                         "one form (per frame three k_walk launches: primary, bounce, any-hit); pipelined = two "
                          "binary frames whose results are copied in bands while they trace; batched-* = two "
-                         "launches of one k_multi batch over the first 16 scenes of the batched workload; "
+                         "launches of one batch over the first 16 scenes of the batched workload (two k_walk launches each); "
                          "probes-* = two probe-field updates of one form (per update one probe-ray and one "
-                         "shadow-ray k_persistent launch; probes-stratified: binary, stratified directions); shade = one quantised frame, then two k_shade_camera "
+                         "shadow-ray k_walk launch; probes-stratified: binary, stratified directions); shade = one quantised frame, then two k_shade_camera "
                          "launches; build = two GPU builds of the 1M-triangle scene")
     args = ap.parse_args()
     if args.profile in ("plain", "wide", "pipelined"):
@@ -1295,18 +1300,20 @@ def main():
                                "(of the rank's band for N > 1), copied into pinned host buffers"},
             "gpu_launches": None, "clocks": clocks,
         }
-        # our kernels per frame: cull, primary trace, secondary generation, kind prefix, secondary trace, ray count
+        # our kernels per frame: cull, primary trace, secondary generation, bounce trace, any-hit trace, ray count
         line["gpu_launches"] = 6 * args.steps * world
         kw = kern[best]
         wide_k = best == "wide"
         line["roofline"] = roofline(
             kw["algorithmic_bytes"], kw["secondary_ms"], l2_gbs, f"frame_secondary_{best}",
-            (f"k_persistent<256, {1 if wide_k else 0}, 0, SecondaryPolicy> "
-             f"({'8-wide' if wide_k else 'binary'} secondary trace of the frame)"),
+            (f"k_walk<256, 0 | 1, {1 if wide_k else 0}, SecondaryPolicy> "
+             f"({'8-wide' if wide_k else 'binary'} secondary trace of the frame: the bounce and the any-hit launch, "
+             "overlapped)"),
             BYTES_WIDE if wide_k else BYTES_PLAIN)
         line["roofline"]["note"] = ("the 11 MB scene is L2-resident: the algorithmic node and triangle bytes are L2 "
                                     "reads, and DRAM carries only the secondary-ray queue (traffic << algorithmic "
-                                    "bytes); the kernel is issue-bound (ncu: instructions and lanes per instruction)")
+                                    "bytes); the any-hit kernel is bound by the L1's data path, the closest-hit kernel by "
+                                    "instruction issue (ncu)")
         line["kernels"] = kern
         if sharding:
             line["sharding"] = sharding

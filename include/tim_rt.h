@@ -132,12 +132,14 @@ int tim_rt_memory_used(tim_rt_ctx *ctx, uint64_t *bytes);
 /* Launch shape of the persistent trace kernels (the knobs the autotuner picks). */
 typedef struct {
     uint32_t block;        /* threads per block: 64, 128 or 256 (default 256) */
-    uint32_t stack_depth;  /* traversal-stack entries per thread; 0 = the scene's tree depth (<= 32) */
-    uint32_t refill_min;   /* a warp fetches new rays once this many of its 32 lanes are idle (1..32);
+    uint32_t stack_depth;  /* traversal-stack entries per thread of the launches that trace both kinds of
+                              rays in one kernel; 0 = the scene's tree depth (<= 32) */
+    uint32_t refill_min;   /* a warp fetches new rays once this many of its 32 lanes are idle (1..32), launches
+                              of any-hit rays alone at half as many again;
                               camera primary rays always refill whole warps (one 8x4-pixel tile) */
     uint32_t ray_sort;     /* batched traces: TIM_RT_SORT_* coherence key the rays are reordered by */
     uint32_t phase_switch; /* 0..31 (default 10): a warp stops its lockstep node rounds and tests the leaves
-                              its lanes hold once only this many lanes still need nodes */
+                              its lanes hold once only this many of 32 lanes under way still need nodes */
 } tim_rt_launch_config;
 #define TIM_RT_SORT_NONE 0u     /* trace in input order */
 #define TIM_RT_SORT_OCTANT 1u   /* group each job's rays by direction octant (stable) */
@@ -233,7 +235,9 @@ int tim_rt_verify_hits(tim_rt_ctx *ctx, tim_rt_scene_id scene, const tim_rt_ray 
 /* ---------------------------------------------------------------- batched multi-scene trace */
 /* Not in the reference, which dispatches one scene per compute pass. A batch is
  * a device-resident table of jobs, each a ray buffer traced against one resident
- * scene; tim_rt_batch_launch traces all of them in ONE persistent kernel launch
+ * scene; tim_rt_batch_launch traces all of them in one persistent kernel launch for
+ * the closest-hit rays and one, overlapped with it, for the any-hit rays (a single one
+ * for both where a scene has a single leaf or was uploaded under a memory budget),
  * whose warps take rays from any job (a lane loads its job's scene when it
  * fetches a ray), so scenes of very uneven size share the GPU without a tail of
  * small launches. Each job's outputs are exactly those of tim_rt_trace_dev on the

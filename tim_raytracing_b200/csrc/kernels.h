@@ -78,7 +78,7 @@ struct CameraBands {
 // [0] pixel work, [1] secondary work, [2, 2 + 26 nb) per-band per-kind counts,
 // [2 + 26 nb, 3 + 52 nb) their prefix (the last entry = secondary rays traced),
 // [3 + 52 nb, 3 + 53 nb) finished rays per band, [3 + 53 nb, 3 + 54 nb) rays per band,
-// [3 + 54 nb] closest-hit secondary work (a launch of its own with the 4-wide tree),
+// [3 + 54 nb] closest-hit secondary work (a launch of its own where the scene has_walk),
 // [4 + 54 nb] generator blocks done.
 uint32_t camera_queue_kinds();
 // Queue segments of a probe update (np*nd slots each): the sun and the 16 light

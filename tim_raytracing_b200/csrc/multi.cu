@@ -1,5 +1,5 @@
-// multi.cu -- batched multi-scene trace: one persistent launch over the rays of
-// many jobs, each traced against its own resident scene, with an optional
+// multi.cu -- batched multi-scene trace: one persistent launch for each kind of ray (or
+// one for both) over the rays of many jobs, each traced against its own resident scene, with an optional
 // coherence sort of the rays (radix sort of a per-ray key) before the trace.
 #include <cuda_runtime.h>
 #include <cub/device/device_radix_sort.cuh>
@@ -69,7 +69,8 @@ __global__ void k_sort_keys(const MultiJob* __restrict__ jobs, uint32_t njobs, u
 }
 
 // One persistent launch over the rays of many jobs, each against its own
-// resident scene. Work item i (or perm[i] when the rays were sorted) belongs to
+// resident scene: the general kernel, for batches of which a scene lacks a form's walks
+// (has_walk). Work item i (or perm[i] when the rays were sorted) belongs to
 // the job j with first[j] <= item < first[j+1]; a lane that refills looks its
 // job up (binary search) and loads that job's scene view, so the lanes of one
 // warp may trace different scenes.

@@ -828,9 +828,10 @@ static void queue_counters(uint32_t* counters, const QueueBands& qb, volatile ui
     g.closest_last = closest_last;
 }
 
-// Traces the queue a generator with these counters left: the rays in one launch, or, with
-// the 4-wide tree, the any-hit rays and the bounce rays in launches of their own, since
-// they walk different trees and a warp of both kinds would walk each with part of its lanes.
+// Traces the queue a generator with these counters left: the rays in one launch, or, where
+// the scene has_walk, the any-hit rays and the bounce rays in launches of their own: in the
+// binary form they walk different trees, of which a warp of both kinds would walk each with
+// part of its lanes, and in both forms an any-hit ray carries half the state.
 static cudaError_t launch_secondary(const SceneView& s, const GenParams& g, uint32_t* counters, uint32_t* err,
                                     cudaStream_t stream, const LaunchConfig& cfg, bool bounces) {
     const uint32_t nb = g.qb.n;
