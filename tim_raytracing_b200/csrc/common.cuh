@@ -9,6 +9,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "grid_cache.h"   // kStackSize
 
 namespace timrt {
 
@@ -23,7 +24,6 @@ constexpr uint32_t kTriBits = 12, kBlasBits = 8, kPrimBits = 8, kLightBits = 4; 
 constexpr uint32_t kLightSphere = 1u;           // primitive_cpp.glsl:8
 constexpr uint32_t kFourCountShift = 27, kFourFirstMask = (1u << kFourCountShift) - 1u;   // 4-wide tree's leaf references
 constexpr uint32_t kFourBytes = 224u, kPairBytes = 112u;   // a node of the 4-wide tree, a child-pair record
-constexpr int kStackSize = 32;                  // the reference's bitstack is 32 bits wide
 
 constexpr uint32_t kQuantNodes = 0x7FFFFFu;   // 8-wide nodes a leaf reference of k_walk can name (bits 8..30)
 

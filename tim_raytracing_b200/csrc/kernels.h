@@ -1,9 +1,9 @@
 // kernels.h -- host-side declarations of the kernel launchers (trace.cu, probes.cu).
 #pragma once
 #include <cstdint>
-#include <mutex>
 #include <cuda_runtime.h>
 #include "common.cuh"
+#include "grid_cache.h"
 #include "../../include/tim_rt.h"
 
 namespace timrt {
@@ -22,28 +22,6 @@ struct LaunchConfig {
     unsigned long long* stats = nullptr;
     // when set, the camera launcher records ev[0..3] around its three phases
     cudaEvent_t* phase_ev = nullptr;
-};
-
-// Grid sizes of one persistent kernel, per device ordinal and stack depth: the
-// occupancy calculator's resident blocks per SM times the device's SM count,
-// computed on first use with the device current (which also sets the kernel's
-// dynamic shared-memory limit in that device's context). Thread-safe.
-struct GridCache {
-    static constexpr int kDevices = 64;
-    std::mutex mu;
-    int blocks[kDevices][kStackSize + 14] = {};   // k_walk: up to 13 words more a thread
-    template <class F>
-    int get(int depth, F compute) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) {
-            cudaGetLastError();
-            dev = -1;
-        }
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev < 0) return compute(0);
-        if (!blocks[dev][depth]) blocks[dev][depth] = compute(dev);
-        return blocks[dev][depth];
-    }
 };
 
 // The kernels' packed knob word: refill threshold (1..32) | phase switch (0..31) << 8.
@@ -119,7 +97,7 @@ size_t multi_sort_temp_bytes(uint32_t total);
 // (k_walk): in the binary form where the scene has those trees, in the 8-wide form where a
 // leaf reference can name all nodes and the stack holds the tree's levels.
 inline bool has_walk(const SceneView& v, bool wide) {
-    return wide ? v.num_wnodes && v.num_wnodes < kQuantNodes && !v.wide_root_is_leaf && v.wide_depth <= kStackSize / 2
+    return wide ? v.num_wnodes && v.num_wnodes < kQuantNodes && !v.wide_root_is_leaf && 2u * v.wide_depth + 2u <= (uint32_t)kWalkStack
                 : v.nodes4 != nullptr;
 }
 // What the jobs of a batch need of the kernels: the deepest tree of each kind, whether

@@ -347,15 +347,17 @@ static int grid_of(GridCache& cache, K* kernel, int depth, int max_depth) {
     });
 }
 
-// Most stack words of an any-hit and a closest-hit ray of k_walk. 24 against 16 words:
+// Most stack words of an any-hit ray of k_walk. 24 against 16 words:
 // the frame's any-hit rays the same, those of a probe update in 1M triangles 1.60
 // against 2.01 ms (16 overflow often enough there for the binary walk to show).
-constexpr int kAnyStack = 24, kWalkStack = kStackSize + 2;
+constexpr int kAnyStack = 24;
+static_assert(kAnyStack <= kWalkStack, "one limit for all walks");
 
 template <int BLOCK, bool ANY, bool QUANT, class Policy>
 static cudaError_t launch_walk_block(const SceneView& s, const Policy& P, uint32_t n_static, uint32_t* counter,
                                      uint32_t* err, int depth, int knobs, int role, int share, cudaStream_t stream) {
     static GridCache cache;
+    static_assert(walk_words<Policy, QUANT> <= kWalkBeside, "GridCache counts on it");
     const int words = depth + walk_words<Policy, QUANT>;
     const int grid = grid_of<BLOCK, Policy>(cache, k_walk<BLOCK, ANY, QUANT, Policy>, words, kWalkStack + walk_words<Policy, QUANT>);
     cudaLaunchConfig_t lc{};
