@@ -18,6 +18,7 @@
 #include <string>
 #include "common.cuh"
 #include "context.h"
+#include "four_stack.h"
 #include "kernels.h"
 
 namespace timrt {
@@ -281,11 +282,16 @@ __global__ void __launch_bounds__(256) k_four_small(In in, const float4* cost, u
     }
 }
 
+// The first node of each level.
+struct Levels { uint32_t count, first[kMaxLevels]; };
+
 __global__ void __launch_bounds__(128) k_four_fill(In in, const float4* cost, const uint32_t* item, const Box* item_e,
-                                                   const uint2* base, uint32_t total, float4* nodes4, uint4* leaf4,
-                                                   uint32_t* tri_leaf4) {
+                                                   const uint2* base, uint32_t total, Levels levels, float4* nodes4,
+                                                   uint4* leaf4, uint32_t* tri_leaf4) {
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= total) return;
+    uint32_t below = 0;   // the levels after w's
+    for (uint32_t lv = 1; lv < levels.count; ++lv) below += w < levels.first[lv] ? 1u : 0u;
     Sub s[4];
     const int n = expand(in, cost, item[w], item_e[w], s);
     uint2 b = base[w];
@@ -299,7 +305,7 @@ __global__ void __launch_bounds__(128) k_four_fill(In in, const float4* cost, co
         ref[k] = 0u;
         if (k >= n) continue;
         if (!(s[k].id & kNidLeafBit)) {
-            ref[k] = b.x++;
+            ref[k] = (below - 1u) << kFourBelowShift | b.x++;   // an inner slot's node is of the next level
             continue;
         }
         const uint32_t nid = s[k].id & kNidMask;
@@ -471,7 +477,7 @@ int build_four(tim_rt_ctx* c, Scene* s, uint64_t num_tris, uint32_t root_left) {
     while (ok && levels < s->depth && h.level[levels + 1u] > h.level[levels]) ++levels;
     float bound[3];
     for (int d = 0; d < 3; ++d) memcpy(&bound[d], &h.bound[d], 4);
-    const bool fits = ok && !h.bad && h.leaves && h.total < (1u << 25) && h.level[levels] == h.total && bound[0] <= 1.099511627776e12f &&
+    const bool fits = ok && !h.bad && h.leaves && h.total <= kFourIndexMask && h.level[levels] == h.total && bound[0] <= 1.099511627776e12f &&
                       bound[1] <= 1.099511627776e12f && bound[2] <= 1.099511627776e12f;   // 2^40
     if (fits) {
         const uint64_t o_pairs = up((uint64_t)kFourBytes * h.total), o_leaf = o_pairs + up((uint64_t)kPairBytes * cap),
@@ -484,7 +490,9 @@ int build_four(tim_rt_ctx* c, Scene* s, uint64_t num_tris, uint32_t root_left) {
             uint4* leaf4 = reinterpret_cast<uint4*>(t + o_leaf);
             uint32_t* tri_leaf4 = reinterpret_cast<uint32_t*>(t + o_tri);
             k_pairs<<<blocks, 256, 0, st>>>(in, pairs);
-            k_four_fill<<<(h.total + 127u) / 128u, 128, 0, st>>>(in, cost, item, item_e, base, h.total, nodes4, leaf4,
+            Levels lv{levels, {}};
+            std::copy(h.level, h.level + levels, lv.first);
+            k_four_fill<<<(h.total + 127u) / 128u, 128, 0, st>>>(in, cost, item, item_e, base, h.total, lv, nodes4, leaf4,
                                                                  tri_leaf4);
             ok = cudaGetLastError() == cudaSuccess;
             v.nodes4 = nodes4;

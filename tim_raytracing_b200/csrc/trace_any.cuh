@@ -11,8 +11,8 @@
 //
 // Node layout (224 B, built by bvh_four.cu):
 //   per axis, 4 x float4: lo[4] hi[4] hi[4] lo[4], one word per slot
-//   uint4   the slots' references: an inner node's index, or a leaf as
-//           bit 31 | triangles << 27 | first triangle (triangles 0: more than
+//   uint4   the slots' references: an inner node's index and the levels below it
+//           (four_stack.h), or a leaf as bit 31 | triangles << 27 | first triangle (triangles 0: more than
 //           15, read from the leaf's record); empty slots have inverted boxes
 //   16 B    unused
 // A ray reads its near and far planes of an axis, in this order, with one 32-byte
@@ -51,6 +51,7 @@
 // instructions. The L1 binds it: 66 % of its data path's cycles, 57 % hits.
 #pragma once
 #include "common.cuh"
+#include "four_stack.h"
 #include "trace_plain.cuh"
 #include "trace_wide.cuh"
 
@@ -117,7 +118,7 @@ __device__ __forceinline__ void any_init(const SceneView& s, TravState& st, uint
     st.top = bottom;
     st.hit = false;
     st.leaf = ok ? 0u : 1u;
-    st.node = ok ? 0u : kAnyIdle;
+    st.node = ok ? (s.depth4 - 1u) << kFourBelowShift : kAnyIdle;
 }
 
 // Eight floats at a 32-byte boundary.
@@ -163,33 +164,60 @@ __device__ __forceinline__ const char* four_refs(const SceneView& s) {
     return reinterpret_cast<const char*>(s.nodes4) + 192u;
 }
 
+// A slot's box test (see the header).
+struct AnyBoxRay { float ix, iy, iz, anx, any_, anz, afx, afy, afz, t; };
+template <class R>
+__device__ __forceinline__ bool any_enters(const R& r, float nx, float fx, float ny, float fy, float nz, float fz) {
+    const float tn = max3f(fmaxf(__fmaf_rn(nx, r.ix, r.anx), __fmaf_rn(ny, r.iy, r.any_)), __fmaf_rn(nz, r.iz, r.anz), 0.0f);
+    const float tf = min3f(fminf(__fmaf_rn(fx, r.ix, r.afx), __fmaf_rn(fy, r.iy, r.afy)), __fmaf_rn(fz, r.iz, r.afz), r.t);
+    return tn < tf;
+}
+
+// The entered slots of a node: any_advance's box tests where the slots don't fit on the
+// stack.
+static __device__ __forceinline__ uint32_t any_slots(AnyBoxRay r, const char* px, const char* py, const char* pz) {
+    float4 nx, fx, ny, fy, nz, fz;
+    load8(px, nx, fx);
+    load8(py, ny, fy);
+    load8(pz, nz, fz);
+    return (any_enters(r, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x) ? 1u : 0u) | (any_enters(r, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y) ? 2u : 0u) |
+           (any_enters(r, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z) ? 4u : 0u) | (any_enters(r, nx.w, fx.w, ny.w, fy.w, nz.w, fz.w) ? 8u : 0u);
+}
+
+// any_advance from a node whose slots don't fit on the stack, or that waits (four_stack.h).
+template <int BLOCK>
+__device__ __forceinline__ void any_advance_tight(TravState& st, const char* refs_base) {
+    if (!(st.node & kFourWaiting)) {
+        const uint64_t off = (uint64_t)(st.node & kFourIndexMask) * kFourBytes;
+        const uint32_t slots = any_slots(AnyBoxRay{st.ix, st.iy, st.iz, st.anx, st.any_, st.anz, st.afx, st.afy, st.afz, st.t},
+                                         st.px + off, st.py + off, st.pz + off);
+        st.node = slots ? four_waiting(st.node, slots) : stack_pop<BLOCK>(st.top);
+        return;
+    }
+    const uint32_t slot = 31u - (uint32_t)__clz((int)(st.node & 15u)), rest = st.node & ~(1u << slot);   // the last of them
+    stack_push<BLOCK>(st.top, rest, (rest & 15u) != 0u);
+    st.node = __ldg(reinterpret_cast<const uint32_t*>(refs_base + (uint64_t)((st.node >> 4) & kFourIndexMask) * kFourBytes) + slot);
+}
+
 // One advance of one lane from the inner node st.node: its slots whose boxes are
 // entered go onto the stack, smallest box first, and the last one is taken. (The
 // entered box nearest first instead: 6 % fewer visits, but 20 more instructions each.)
 template <int BLOCK>
-__device__ __forceinline__ void any_advance(TravState& st, const char* refs_base, uint32_t limit) {
-    if (st.top > limit) {   // more slots wait than the stack has room for: the binary walk
-        st.leaf = 1u;
-        st.node = kAnyIdle;
+__device__ __forceinline__ void any_advance(TravState& st, const char* refs_base, uint32_t near, uint32_t bottom, int sdepth) {
+    if (st.top >= near && !four_fits(st.top, st.node, bottom, sdepth, 4u * BLOCK)) {
+        any_advance_tight<BLOCK>(st, refs_base);
         return;
     }
-    const uint64_t off = (uint64_t)st.node * kFourBytes;
+    const uint64_t off = (uint64_t)(st.node & kFourIndexMask) * kFourBytes;
     float4 nx, fx, ny, fy, nz, fz;
     load8(st.px + off, nx, fx);
     load8(st.py + off, ny, fy);
     load8(st.pz + off, nz, fz);
     const uint4 ref = __ldg(reinterpret_cast<const uint4*>(refs_base + off));
-    const float nxs[4] = {nx.x, nx.y, nx.z, nx.w}, nys[4] = {ny.x, ny.y, ny.z, ny.w}, nzs[4] = {nz.x, nz.y, nz.z, nz.w};
-    const float fxs[4] = {fx.x, fx.y, fx.z, fx.w}, fys[4] = {fy.x, fy.y, fy.z, fy.w}, fzs[4] = {fz.x, fz.y, fz.z, fz.w};
-    const uint32_t refs[4] = {ref.x, ref.y, ref.z, ref.w};
-#pragma unroll
-    for (uint32_t k = 0; k < 4u; ++k) {
-        const float tn = max3f(fmaxf(__fmaf_rn(nxs[k], st.ix, st.anx), __fmaf_rn(nys[k], st.iy, st.any_)),
-                               __fmaf_rn(nzs[k], st.iz, st.anz), 0.0f);
-        const float tf = min3f(fminf(__fmaf_rn(fxs[k], st.ix, st.afx), __fmaf_rn(fys[k], st.iy, st.afy)),
-                               __fmaf_rn(fzs[k], st.iz, st.afz), st.t);
-        stack_push<BLOCK>(st.top, refs[k], tn < tf);
-    }
+    stack_push<BLOCK>(st.top, ref.x, any_enters(st, nx.x, fx.x, ny.x, fy.x, nz.x, fz.x));
+    stack_push<BLOCK>(st.top, ref.y, any_enters(st, nx.y, fx.y, ny.y, fy.y, nz.y, fz.y));
+    stack_push<BLOCK>(st.top, ref.z, any_enters(st, nx.z, fx.z, ny.z, fy.z, nz.z, fz.z));
+    stack_push<BLOCK>(st.top, ref.w, any_enters(st, nx.w, fx.w, ny.w, fy.w, nz.w, fz.w));
     st.node = stack_pop<BLOCK>(st.top);
 }
 

@@ -103,8 +103,7 @@ constexpr int walk_threads = filters<Policy>::value || (QUANT && !ANY) ? 768 : 1
 // the 8-wide form (QUANT) both on the quantised one (trace_quant.cuh). The same
 // persistent loop, with the ray's place in st.node alone -- an inner node, a leaf, or
 // kAnyIdle, which is also the lowest word of its stack, so that popping it ends the
-// walk. sdepth: stack words per thread; an any-hit ray that would need more takes the
-// plain binary walk, no other ray ever does.
+// walk. sdepth: stack words per thread, as many as any ray needs.
 //
 // A batch of both kinds is two launches (kPairFirst, kPairSecond) that may overlap: the
 // first lets the second start as soon as its own blocks leave room, so that the second's
@@ -142,7 +141,7 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOC
     // and probe fields (16 to 22 lanes) are faster on their own lanes, 0.92 against 0.97 ms.
     constexpr bool kSpread = !ANY || filters<Policy>::value;
     const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(stk);
-    const uint32_t limit = bottom + ((uint32_t)sdepth - 5u) * BLOCK * 4u;   // an any-hit visit pushes up to four words
+    const uint32_t near = four_near(bottom, sdepth, (int)s.depth4, 4u * BLOCK);   // any-hit rays (four_stack.h)
 
     TravState st;
     st.node = kAnyIdle;
@@ -225,7 +224,7 @@ __global__ void __launch_bounds__(BLOCK, walk_threads<Policy, ANY, QUANT> / BLOC
                                    : ANY                      ? four_refs(s)
                                                               : pair_refs(s);
                 if (QUANT) quant_advance<BLOCK, ANY>(st, refs, bottom);
-                else if (ANY) any_advance<BLOCK>(st, refs, limit);
+                else if (ANY) any_advance<BLOCK>(st, refs, near, bottom, sdepth);
                 else pair_advance<BLOCK>(st, refs, dir);
             }
         }
@@ -347,10 +346,6 @@ static int grid_of(GridCache& cache, K* kernel, int depth, int max_depth) {
     });
 }
 
-// Most stack words of an any-hit ray of k_walk. 24 against 16 words:
-// the frame's any-hit rays the same, those of a probe update in 1M triangles 1.60
-// against 2.01 ms (16 overflow often enough there for the binary walk to show).
-constexpr int kAnyStack = 24;
 static_assert(kAnyStack <= kWalkStack, "one limit for all walks");
 
 template <int BLOCK, bool ANY, bool QUANT, class Policy>
@@ -388,8 +383,7 @@ static cudaError_t launch_walk(const SceneView& s, const Policy& P, uint32_t n_s
     if (QUANT) {
         depth = 2 * (int)s.wide_depth + 2;
     } else if (ANY) {
-        depth = 3 * (int)s.depth4 + 2;
-        depth = depth < 6 ? 6 : (depth > kAnyStack ? kAnyStack : depth);
+        depth = four_words((int)s.depth4);
     }
     // any-hit rays of one origin's neighbourhood profit more from starting together (they
     // read the same nodes; the L1 binds this walk): 16 -> 24 idle lanes, 0.81 -> 0.73 ms
