@@ -214,7 +214,8 @@ int tim_rt_scene_bytes(tim_rt_ctx *ctx, tim_rt_scene_id scene, uint64_t *bytes);
  * bary (optional): (u, v) of the accepted Moller-Trumbore hit, (0, 0) otherwise. */
 int tim_rt_trace(tim_rt_ctx *ctx, tim_rt_scene_id scene, const tim_rt_ray *rays, uint32_t n, uint32_t mode,
                  uint32_t *hit, uint32_t *leaf_nid, float *bary, tim_rt_stats *stats);
-/* Device-pointer form of tim_rt_trace; stream-ordered, no synchronisation. */
+/* Device-pointer form of tim_rt_trace; stream-ordered, no synchronisation. Up to 4,096
+ * calls of a context may be in flight at once, over all streams. */
 int tim_rt_trace_dev(tim_rt_ctx *ctx, tim_rt_scene_id scene, const tim_rt_ray *d_rays, uint32_t n, uint32_t mode,
                      uint32_t *d_hit, uint32_t *d_leaf_nid, float *d_bary, void *cuda_stream);
 

@@ -242,6 +242,7 @@ int tim_rt_create(int device, uint64_t mem_budget_bytes, tim_rt_ctx** out) {
     TIMRT_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->band_flags_dev), c->band_flags, 0));
     int rc = dev_alloc(c.get(), c->counters, 4ull * kCounterWords);
     if (rc) return rc;
+    TIMRT_CUDA(cudaMalloc(reinterpret_cast<void**>(&c->ring_mem), 4ull * kRingWords));
     if ((rc = dev_alloc(c.get(), c->dstats, 256))) return rc;   // 16 counter words + 16 verification words
     if ((rc = dev_alloc(c.get(), c->ray_acc, 16))) return rc;
     TIMRT_CUDA(cudaMemset(c->counters.ptr, 0, 4ull * kCounterWords));
@@ -270,6 +271,7 @@ int tim_rt_destroy(tim_rt_ctx* c) {
                       &c->p_out, &c->p_nid, &c->p_irr, &c->p_sh16, &c->p_sh32, &c->p_octa, &c->sh_out, &c->sh_f32, &c->bld, &c->ray_acc,
                       &c->band_ctr})
         dev_free(c, *b);
+    cudaFree(c->ring_mem);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : c->pev)
@@ -526,7 +528,7 @@ int tim_rt_trace_dev(tim_rt_ctx* c, tim_rt_scene_id id, const tim_rt_ray* d_rays
     }
     if (n == 0) return TIM_RT_OK;
     cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : c->stream;
-    uint32_t* ctr = static_cast<uint32_t*>(c->counters.ptr) + kRingBase + 2u * (c->ring++ % (kRingSize / 2u));
+    uint32_t* ctr = c->ring_mem + ring_word(c->ring++);
     uint32_t* err = static_cast<uint32_t*>(c->counters.ptr) + kErrWord;
     TIMRT_CUDA(cudaMemsetAsync(ctr, 0, 8, st));
     TIMRT_CUDA(launch_trace_batch(s->view, d_rays, n, mode, d_hit, d_nid, d_bary, ctr, err, st,

@@ -8,6 +8,7 @@
 #include <set>
 #include <string>
 #include <vector>
+#include "counter_ring.h"
 #include "internal.h"
 #include "kernels.h"
 
@@ -46,7 +47,8 @@ struct tim_rt_ctx {
     uint32_t next_id = 1;
     // scratch
     DevBuf rays, hits, nid, bary;
-    DevBuf counters;            // [0..63] per-call work counters, [64] device error word, ring after
+    DevBuf counters;            // [0..63] per-call work counters, [64] device error word
+    uint32_t* ring_mem = nullptr;   // tim_rt_trace_dev's counters (counter_ring.h)
     uint32_t ring = 0;
     DevBuf cam_out, cam_bounce, cam_nid, q_rays, q_pixel, tiles_counts, tiles_lists;
     DevBuf dstats;              // [0..15] u64 work counters of the counting kernels, [16..20] verification
@@ -82,9 +84,8 @@ struct tim_rt_batch {
 
 namespace timrt {
 
-constexpr uint32_t kCounterWords = 64 + 1 + 4096;   // fixed counters, error word, trace_dev ring
+constexpr uint32_t kCounterWords = 64 + 1;   // fixed counters, error word
 constexpr uint32_t kErrWord = 64;
-constexpr uint32_t kRingBase = 65, kRingSize = 4096;
 
 // Device allocation admitted against the context's budget.
 int dev_alloc(tim_rt_ctx* c, DevBuf& b, uint64_t bytes);
