@@ -1229,7 +1229,7 @@ int tim_rt_autotune_batch(tim_rt_ctx* c, tim_rt_batch* b, uint32_t flags, uint32
         }
         for (int sd : {0, 32}) {
             LaunchConfig cand = best;
-            if (cand.stack_depth == sd) continue;
+            if (cand.stack_depth == sd || b->needs.walk[best_wide]) continue;   // such launches have no use for it
             cand.stack_depth = sd;
             consider(cand, best_wide);
         }
