@@ -285,8 +285,6 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n = items_of(P, n_static);
     const uint32_t root = s.num_nodes == 1u ? kNidLeafBit : 0u;   // baseRaytracingPass.glsl:20
-    uint32_t* pool = stack_mem + (size_t)sdepth * BLOCK + (threadIdx.x & ~31u);   // filters<Policy> only
-    uint32_t used = 0, have = 0;
 
     TravState st;
     st.done = true;
@@ -329,19 +327,14 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1024 / BLOCK) k_pe
             }
             if constexpr (finishes<Policy>::value) P.finished(stored, st.slot2);
             if (!exhausted) {
-                const uint32_t need = idle;
-                if constexpr (filters<Policy>::value) {
-                    refill_filtered(P, n, counter, pool, need, used, have, exhausted, start);
-                } else {
-                    const int leader = __ffs(need) - 1;
-                    uint32_t base = 0;
-                    if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(need));
-                    base = __shfl_sync(0xFFFFFFFFu, base, leader);
-                    if ((uint64_t)base + (uint32_t)__popc(need) >= n) exhausted = true;
-                    if (!active) {
-                        const uint32_t my = base + __popc(need & lanemask_lt());
-                        if (my < n) start(my);
-                    }
+                const int leader = __ffs(idle) - 1;
+                uint32_t base = 0;
+                if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(idle));
+                base = __shfl_sync(0xFFFFFFFFu, base, leader);
+                if ((uint64_t)base + (uint32_t)__popc(idle) >= n) exhausted = true;
+                if (!active) {
+                    const uint32_t my = base + __popc(idle & lanemask_lt());
+                    if (my < n) start(my);
                 }
             }
         }
