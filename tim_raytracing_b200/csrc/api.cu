@@ -167,7 +167,7 @@ int probe_plan(Scene* s, const tim_rt_probe_desc* desc, uint32_t probe_begin, ui
         set_error(w + ": scene was uploaded without TIM_RT_UPLOAD_QUANT8");
         return TIM_RT_EUNSUPPORTED;
     }
-    if (!s->nrm.ptr) {
+    if (!s->view.nrm) {
         set_error(w + ": the lit value needs vertex normals (upload with nrm)");
         return TIM_RT_EINVAL;
     }
@@ -324,6 +324,40 @@ int tim_rt_memory_used(tim_rt_ctx* c, uint64_t* bytes) {
     return TIM_RT_OK;
 }
 
+}  // extern "C"
+namespace {
+
+// Bytes up to which a scene of few nodes is brought over as one.
+constexpr uint64_t kSmallUpload = 1u << 20;
+
+// Least and largest coordinates (a NaN counts where it is the first vertex's). Four
+// vertices at a time, in the order of memory: twelve chains of minima where one an axis
+// took 110 of the 360 us of an upload of 10,000 triangles.
+void vertex_bounds(const float* pos, uint32_t n, float bounds[6]) {
+    float lo[12], hi[12];
+    for (int k = 0; k < 12; ++k) lo[k] = hi[k] = pos[k % 3];
+    uint64_t i = 0;
+    const uint64_t words = 3ull * n;
+    for (; i + 12 <= words; i += 12)
+        for (int k = 0; k < 12; ++k) {
+            const float x = pos[i + k];
+            lo[k] = x < lo[k] ? x : lo[k];
+            hi[k] = hi[k] < x ? x : hi[k];
+        }
+    for (; i < words; ++i) {
+        const int k = (int)(i % 3);
+        lo[k] = std::min(lo[k], pos[i]);
+        hi[k] = std::max(hi[k], pos[i]);
+    }
+    for (int k = 0; k < 12; ++k) {
+        bounds[k % 3] = k < 3 ? lo[k] : std::min(bounds[k % 3], lo[k]);
+        bounds[3 + k % 3] = k < 3 ? hi[k] : std::max(bounds[3 + k % 3], hi[k]);
+    }
+}
+
+}  // namespace
+extern "C" {
+
 int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, const uint32_t ranges[7][2],
                       const float* pos, const float* nrm, const float* uv, uint32_t max_vertex, uint32_t num_vertex,
                       const tim_rt_push_constants* pc, uint32_t flags, tim_rt_scene_id* out) {
@@ -356,44 +390,92 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
         }
         s->blas_roots_ok = ok;
     }
-    for (int a = 0; a < 3; ++a) {
-        float lo = pos[a], hi = pos[a];
-        for (uint32_t i = 1; i < num_vertex; ++i) {
-            lo = std::min(lo, pos[3ull * i + a]);
-            hi = std::max(hi, pos[3ull * i + a]);
-        }
-        s->bounds[a] = lo;
-        s->bounds[3 + a] = hi;
-    }
-    WideHost wh;
-    if (flags & TIM_RT_UPLOAD_QUANT8) {
-        if (pc->numBlas) {
-            set_error("tim_rt_upload_bvh: the 8-wide form does not support BLAS instances");
-            return TIM_RT_EUNSUPPORTED;
-        }
-        if (!build_wide(blob, ranges, pc->numNodes, pos, wh, err)) {
-            set_error("tim_rt_upload_bvh: 8-wide build: " + err);
-            return TIM_RT_EUNSUPPORTED;
-        }
+    vertex_bounds(pos, num_vertex, s->bounds);
+    if ((flags & TIM_RT_UPLOAD_QUANT8) && pc->numBlas) {
+        set_error("tim_rt_upload_bvh: the 8-wide form does not support BLAS instances");
+        return TIM_RT_EUNSUPPORTED;
     }
     auto fail = [&](int code) {
         for (DevBuf* b : {&s->blob, &s->pos, &s->nrm, &s->uv, &s->wnodes, &s->wtris, &s->wnid, &s->ptris, &s->pleaf, &s->trees}) dev_free(c, *b);
         return code;
     };
-    if ((rc = dev_alloc(c, s->blob, n_bytes))) return fail(rc);
-    if ((rc = dev_alloc(c, s->pos, 12ull * max_vertex))) return fail(rc);
-    if (nrm && (rc = dev_alloc(c, s->nrm, 12ull * max_vertex))) return fail(rc);
-    if (uv && (rc = dev_alloc(c, s->uv, 8ull * max_vertex))) return fail(rc);
-    if ((rc = dev_alloc(c, s->pleaf, 16ull * pc->numNodes))) return fail(rc);
-    if (tris && (rc = dev_alloc(c, s->ptris, 48ull * tris))) return fail(rc);
-    if (cudaMemcpyAsync(s->blob.ptr, blob, n_bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-        cudaMemcpyAsync(s->pos.ptr, pos, 12ull * num_vertex, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-        (nrm && cudaMemcpyAsync(s->nrm.ptr, nrm, 12ull * num_vertex, cudaMemcpyHostToDevice, c->stream) != cudaSuccess) ||
-        (uv && cudaMemcpyAsync(s->uv.ptr, uv, 8ull * num_vertex, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)) {
-        set_error("tim_rt_upload_bvh: host-to-device copy failed");
-        return fail(TIM_RT_EDEVICE);
+    uint32_t root_left;   // the root's first child
+    std::memcpy(&root_left, blob + ranges[TIM_RT_RANGE_NODE][0] + 8, 4);
+    root_left &= 0x3FFFFFFFu;
+    SceneView& v = s->view;
+    auto set_blob = [&](const uint8_t* d) {
+        v.nodes = reinterpret_cast<const float4*>(d + ranges[TIM_RT_RANGE_NODE][0]);
+        v.leaf = reinterpret_cast<const uint32_t*>(d + ranges[TIM_RT_RANGE_LEAF][0]);
+        v.lights = reinterpret_cast<const float*>(d + ranges[TIM_RT_RANGE_LIGHT][0]);
+        v.blas = reinterpret_cast<const float*>(d + ranges[TIM_RT_RANGE_BLAS][0]);
+        v.materials = reinterpret_cast<const float*>(d + ranges[TIM_RT_RANGE_MAT][0]);
+    };
+    TreeBuild trees(c, s.get(), tris);
+    HostTrees ht;
+    RawVec<uint8_t> image;   // of a small scene
+    bool small = host_trees(c, blob, ranges, *pc, depth, tris, ht);
+    if (small) {
+        // few nodes: everything in one allocation, brought over by one copy
+        const uint64_t vec = 12ull * max_vertex, o_pos = up256(n_bytes), o_nrm = o_pos + up256(vec),
+                       o_uv = o_nrm + (nrm ? up256(vec) : 0ull), o_img = o_uv + (uv ? up256(8ull * max_vertex) : 0ull),
+                       o_tris = up256(o_img + ht.image.size());
+        const std::string last_error = g_last_error;
+        small = o_tris <= kSmallUpload && dev_alloc(c, s->blob, o_tris + 48ull * tris) == TIM_RT_OK;
+        if (small) {
+            image.resize(o_img + ht.image.size());
+            std::memcpy(image.data(), blob, n_bytes);
+            std::memcpy(image.data() + o_pos, pos, 12ull * num_vertex);
+            if (nrm) std::memcpy(image.data() + o_nrm, nrm, 12ull * num_vertex);
+            if (uv) std::memcpy(image.data() + o_uv, uv, 8ull * num_vertex);
+            std::memcpy(image.data() + o_img, ht.image.data(), ht.image.size());
+            uint8_t* d = static_cast<uint8_t*>(s->blob.ptr);
+            set_blob(d);
+            v.pos = reinterpret_cast<const float*>(d + o_pos);
+            v.nrm = nrm ? reinterpret_cast<const float*>(d + o_nrm) : nullptr;
+            v.ptris = reinterpret_cast<const float4*>(d + o_tris);
+            ht.place(d + o_img, root_left, v);
+            if (cudaMemcpyAsync(d, image.data(), image.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess) {
+                set_error("tim_rt_upload_bvh: host-to-device copy failed");
+                return fail(TIM_RT_EDEVICE);
+            }
+        } else {
+            set_error(last_error);
+        }
     }
+    v.num_nodes = pc->numNodes;
+    v.num_lights = pc->numLights;
+    v.leaf_words = ranges[TIM_RT_RANGE_LEAF][1] / 4u;
+    v.num_vertex = num_vertex;
+    v.depth = depth;
+    if (!small) {
+        if ((rc = dev_alloc(c, s->blob, n_bytes))) return fail(rc);
+        if ((rc = dev_alloc(c, s->pos, 12ull * max_vertex))) return fail(rc);
+        if (nrm && (rc = dev_alloc(c, s->nrm, 12ull * max_vertex))) return fail(rc);
+        if (uv && (rc = dev_alloc(c, s->uv, 8ull * max_vertex))) return fail(rc);
+        if ((rc = dev_alloc(c, s->pleaf, 16ull * pc->numNodes))) return fail(rc);
+        if (tris && (rc = dev_alloc(c, s->ptris, 48ull * tris))) return fail(rc);
+        set_blob(static_cast<const uint8_t*>(s->blob.ptr));
+        v.pos = static_cast<const float*>(s->pos.ptr);
+        v.nrm = static_cast<const float*>(s->nrm.ptr);
+        v.pleaf = static_cast<const uint4*>(s->pleaf.ptr);
+        v.ptris = static_cast<const float4*>(s->ptris.ptr);
+        // the trees are built from the image while the vertices come over on the copy stream
+        if (cudaMemcpyAsync(s->blob.ptr, blob, n_bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+            trees.begin() != cudaSuccess ||
+            cudaMemcpyAsync(s->pos.ptr, pos, 12ull * num_vertex, cudaMemcpyHostToDevice, c->cstream) != cudaSuccess ||
+            (nrm && cudaMemcpyAsync(s->nrm.ptr, nrm, 12ull * num_vertex, cudaMemcpyHostToDevice, c->cstream) != cudaSuccess) ||
+            (uv && cudaMemcpyAsync(s->uv.ptr, uv, 8ull * num_vertex, cudaMemcpyHostToDevice, c->cstream) != cudaSuccess) ||
+            cudaEventRecord(c->copy_ev, c->cstream) != cudaSuccess || cudaStreamWaitEvent(c->stream, c->copy_ev, 0) != cudaSuccess) {
+            set_error("tim_rt_upload_bvh: host-to-device copy failed");
+            return fail(TIM_RT_EDEVICE);
+        }
+    }
+    WideHost wh;
     if (flags & TIM_RT_UPLOAD_QUANT8) {
+        if (!build_wide(blob, ranges, pc->numNodes, pos, wh, err)) {
+            set_error("tim_rt_upload_bvh: 8-wide build: " + err);
+            return fail(TIM_RT_EUNSUPPORTED);
+        }
         if ((rc = dev_alloc(c, s->wnodes, 4ull * wh.nodes.size()))) return fail(rc);
         if ((rc = dev_alloc(c, s->wtris, 4ull * wh.tris.size()))) return fail(rc);
         if ((rc = dev_alloc(c, s->wnid, 4ull * wh.tri_leaf.size()))) return fail(rc);
@@ -405,36 +487,17 @@ int tim_rt_upload_bvh(tim_rt_ctx* c, const void* bvh_bytes, uint64_t n_bytes, co
         }
         s->has_wide = true;
     }
-    const uint8_t* d = static_cast<const uint8_t*>(s->blob.ptr);
-    SceneView& v = s->view;
-    v.nodes = reinterpret_cast<const float4*>(d + ranges[TIM_RT_RANGE_NODE][0]);
-    v.leaf = reinterpret_cast<const uint32_t*>(d + ranges[TIM_RT_RANGE_LEAF][0]);
-    v.pos = static_cast<const float*>(s->pos.ptr);
-    v.nrm = static_cast<const float*>(s->nrm.ptr);
-    v.lights = reinterpret_cast<const float*>(d + ranges[TIM_RT_RANGE_LIGHT][0]);
-    v.blas = reinterpret_cast<const float*>(d + ranges[TIM_RT_RANGE_BLAS][0]);
-    v.materials = reinterpret_cast<const float*>(d + ranges[TIM_RT_RANGE_MAT][0]);
-    v.num_nodes = pc->numNodes;
-    v.num_lights = pc->numLights;
-    v.leaf_words = ranges[TIM_RT_RANGE_LEAF][1] / 4u;
-    v.num_vertex = num_vertex;
-    v.depth = depth;
     v.wide_depth = wh.max_depth;
     v.wnodes = static_cast<const uint4*>(s->wnodes.ptr);
     v.wtris = static_cast<const float4*>(s->wtris.ptr);
     v.wtri_leaf = static_cast<const uint4*>(s->wnid.ptr);
     v.num_wnodes = s->has_wide ? wh.num_nodes : 0u;
     v.wide_root_is_leaf = wh.root_is_leaf;
-    v.pleaf = static_cast<const uint4*>(s->pleaf.ptr);
-    v.ptris = static_cast<const float4*>(s->ptris.ptr);
-    if (build_leaf_tris(s.get(), c->stream) != cudaSuccess) {
+    if (!small && (rc = trees.end(root_left))) return fail(rc);
+    if (fill_leaf_tris(s.get(), c->stream) != cudaSuccess) {
         set_error("tim_rt_upload_bvh: building the leaf triangles failed");
         return fail(TIM_RT_EDEVICE);
     }
-    uint32_t root_left;   // the root's first child
-    std::memcpy(&root_left, blob + ranges[TIM_RT_RANGE_NODE][0] + 8, 4);
-    root_left &= 0x3FFFFFFFu;
-    if ((rc = build_four(c, s.get(), tris, root_left))) return fail(rc);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
         set_error("tim_rt_upload_bvh: stream synchronisation failed");
         return fail(TIM_RT_EDEVICE);
@@ -742,7 +805,7 @@ static int shade_check(Scene* s, const tim_rt_pass_data* pd, uint32_t flags, con
             return TIM_RT_EINVAL;
         }
     }
-    if (!s->nrm.ptr) {
+    if (!s->view.nrm) {
         set_error(w + ": the lit value needs vertex normals (upload with nrm)");
         return TIM_RT_EINVAL;
     }

@@ -93,13 +93,46 @@ void dev_free(tim_rt_ctx* c, DevBuf& b);
 // Makes the context's device current; TIM_RT_EINVAL for a null context.
 int check_ctx(tim_rt_ctx* c);
 Scene* find_scene(tim_rt_ctx* c, tim_rt_scene_id id);
-// Fills the scene's leaf triangles (view.pleaf, view.ptris) from its uploaded nodes, leaf
-// data and positions, on the context's stream.
-cudaError_t build_leaf_tris(const Scene* s, cudaStream_t stream);
-// Builds the 4-wide tree of a scene's any-hit rays and the child-pair records of its closest-hit rays from its uploaded arrays (view
-// filled up to ptris; num_tris leaf triangles). A scene the form does not cover is
-// left without it (TIM_RT_OK, view.nodes4 null). Synchronous.
-int build_four(tim_rt_ctx* c, Scene* s, uint64_t num_tris, uint32_t root_left);
+// Offsets of a scene's trees in one buffer, nodes4 first.
+struct TreePlan {
+    uint64_t pairs = 0, leaf4 = 0, tri_leaf4 = 0, bytes = 0;
+    TreePlan() = default;
+    TreePlan(uint64_t nodes4, uint64_t inner, uint64_t leaves, uint64_t tris);
+};
+inline uint64_t up256(uint64_t x) { return (x + 255ull) & ~255ull; }
+
+// The GPU's build of a scene's leaf records (view.pleaf), the 4-wide tree of its any-hit rays
+// and the child-pair records of its closest-hit rays, on the context's stream, from its
+// uploaded nodes and leaf data (view.nodes, view.leaf, view.pleaf; num_tris leaf triangles).
+// Between begin and end nothing may touch ptris. A scene the trees do not cover is left
+// without them (view.nodes4 null).
+struct TreeBuild {
+    tim_rt_ctx* c;
+    Scene* s;
+    uint64_t num_tris;
+    uint8_t* tmp = nullptr;   // the scratch of a build under way
+    DevBuf scratch;
+    uint64_t o[4] = {};
+    uint32_t cap = 0;
+    TreeBuild(tim_rt_ctx* ctx, Scene* scene, uint64_t tris) : c(ctx), s(scene), num_tris(tris) {}
+    ~TreeBuild();
+    cudaError_t begin();               // launches only
+    int end(uint32_t root_left);       // waits for them, allocates and fills the trees
+};
+// Fills the leaf triangles (view.ptris) from the leaf records and positions, on a stream.
+cudaError_t fill_leaf_tris(const Scene* s, cudaStream_t stream);
+// The same leaf records and trees made on the host, for scenes of few nodes: an image for the
+// device. False where the scene has more nodes, or the trees do not cover it.
+struct HostTrees {
+    RawVec<uint8_t> image;   // the leaf records, and from trees_at the trees
+    uint64_t trees_at = 0;
+    TreePlan plan;
+    uint32_t levels = 0;
+    float bound[3] = {};
+    void place(const uint8_t* d, uint32_t root_left, SceneView& v) const;   // the image's device copy
+};
+bool host_trees(const tim_rt_ctx* c, const uint8_t* blob, const uint32_t ranges[7][2], const tim_rt_push_constants& pc,
+                uint32_t depth, uint64_t tris, HostTrees& out);
 // Stops a server's worker and releases its device memory (context teardown).
 void server_shutdown(tim_rt_ctx* c, tim_rt_server* s);
 
