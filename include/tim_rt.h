@@ -160,9 +160,9 @@ int tim_rt_measure_l2_bandwidth(int device, uint64_t bytes, int passes, float *g
  * The buffers are validated (ranges inside the buffer, node children and leaf
  * offsets in range, vertex indices < num_vertex) before anything is launched;
  * a malformed buffer returns TIM_RT_EINVAL. A context without a memory budget also
- * builds, on the GPU, the trees its binary-form rays walk (same results): a 4-wide tree
+ * builds the trees its binary-form rays walk (same results): a 4-wide tree
  * over the image's leaves for any-hit rays and records of child pairs for closest-hit
- * rays, about 150 B per leaf; a scene that has BLAS instances, or no room for them, is
+ * rays, about 250 B per leaf; a scene that has BLAS instances, or no room for them, is
  * traced through its own nodes, as in a context with a budget. */
 int tim_rt_upload_bvh(tim_rt_ctx *ctx, const void *bvh_bytes, uint64_t n_bytes, const uint32_t ranges[7][2],
                       const float *pos, const float *nrm, const float *uv, uint32_t max_vertex, uint32_t num_vertex,

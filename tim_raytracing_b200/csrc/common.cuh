@@ -50,7 +50,7 @@ struct SceneView {
     uint32_t wide_root_is_leaf; // scene is a single leaf
     // the plain form's leaf-triangle copy (null: read the reference's leaf data and
     // positions directly, as the allocation-free entry point does)
-    const uint4* pleaf;         // per node: (first triangle, leaf header, leaf-data offset, 0)
+    const uint4* pleaf;         // per node: (first triangle, leaf header, leaf-data offset, unused)
     const float4* ptris;        // 3 x float4 per leaf triangle: (p0, vo) (e1, i01) (e2, i2m)
     // the 4-wide tree of the any-hit rays over the leaves of ptris (trace_any.cuh; null: none)
     const float4* nodes4;       // 14 x float4 per node

@@ -21,8 +21,8 @@ struct DevBuf {
 
 struct Scene {
     DevBuf blob, pos, nrm, uv, wnodes, wtris, wnid;
-    DevBuf trees;          // the binary form's trees: nodes4, pairs, leaf4, tri_leaf4 of the view (build_four)
-    DevBuf ptris, pleaf;   // the leaf triangles by node (build_leaf_tris)
+    DevBuf trees;          // the binary form's trees: nodes4, pairs, leaf4, tri_leaf4 of the view (TreeBuild)
+    DevBuf ptris, pleaf;   // the leaf triangles, and each node's (TreeBuild, fill_leaf_tris)
     SceneView view{};
     uint32_t ranges[7][2];
     tim_rt_push_constants pc{};

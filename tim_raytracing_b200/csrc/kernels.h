@@ -39,9 +39,10 @@ cudaError_t launch_trace_batch(const SceneView& s, const tim_rt_ray* rays, uint3
 // band b covers rows [row[b], row[b+1]) (row[0] = 0, row[n] = H, the others
 // multiples of 4). Primary rays and their secondary rays are generated for the
 // whole frame at once, each band's secondary rays in its own part of the queue,
-// and the one secondary launch takes the bands in order, counting finished rays
-// per band and setting flags[b] (host memory the device writes) once band b's
-// records are final, so a host thread can start that band's copy.
+// and the secondary launch, or the pair of one for each kind of ray (has_walk), takes the
+// bands in order, counting finished rays per band and setting flags[b] (host memory the
+// device writes) once band b's records are final, so a host thread can start that band's
+// copy.
 constexpr uint32_t kMaxCamBands = 8;
 struct CameraBands {
     uint32_t n;

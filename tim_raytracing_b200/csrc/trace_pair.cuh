@@ -8,7 +8,8 @@
 // takes per axis and box and the per-node leaf record:
 //   per axis, 2 x float4: (lo[2], hi[2]) (hi[2], lo[2]), one word per child
 //   ref[2]      the record of an inner child's children, or a leaf as
-//               bit 31 | triangles << 27 | first triangle (triangles 0: more than 15)
+//               bit 31 | triangles << 27 | first triangle (triangles 0: more than 15, or
+//               none where all bits of the first triangle are set)
 //   8 B         unused
 // A pair of children l, l + 1 is stored at index l / 2: pairs are disjoint, so no two
 // share one. A ray reads its near and far planes of an axis with one 16-byte load,
@@ -25,7 +26,7 @@
 //                                   ->  child 0 first; the latter mirrored, child 1
 // (e and tiny exceed four times the error of the values and of the tests). Entries
 // set by planes both children share are equal in the reference too: child 0 first.
-// Anything else is decided by the reference's divisions (exact_children). A ray
+// Anything else is decided by the reference's divisions (pair_exact). A ray
 // outside the ranges has tiny = +inf and takes them at every node.
 #pragma once
 #include "common.cuh"
