@@ -984,13 +984,16 @@ __device__ __forceinline__ uint32_t probe_sample(const ProbeArgs& d, uint32_t i,
     return pl * d.nd + r;
 }
 
-// Work item i of the probe-ray trace. It is probe-major like the generator,
-// except under TIM_RT_PROBE_OCTA (the directions are the octahedral grid), where it
-// is direction-major (r = i / np: a warp traces one direction from 32
-// neighbouring probes; trace_dir_major is set from that flag). Measured
-// per update on the 1M-triangle scene, 32x32x8 probes x 256 directions: the
-// octahedral set takes 4.17 ms this way against 4.28 ms probe-major, the
-// stratified set 3.71 ms probe-major against 3.85 ms direction-major.
+// Work item i of the probe-ray trace. It is probe-major like the generator, except for
+// octahedral directions (TIM_RT_PROBE_OCTA) on the 8-wide walk and in the general kernel,
+// where it is direction-major (r = i / np: a warp traces one direction from 32
+// neighbouring probes).
+// An update of 32x32x8 probes x 256 directions, direction-major against probe-major:
+// binary walk, 1M triangles, octahedral 3.25 / 3.05 ms, stratified 2.76 / 2.63; octahedral
+// on 2,000 to 300,000 triangles and 64 to 8,192 probes 1 to 17 % in favour of the latter;
+// on the 8-wide walk, 300,000 triangles, 3.48 / 4.48 ms (20,000: 2.51 / 2.81; fields of 64
+// to 384 probes 6 to 43 % the other way, 0.9 / 1.2 ms at most); general kernel, 1M
+// triangles, 4.17 / 4.28 ms.
 __device__ __forceinline__ uint32_t probe_trace_item(const ProbeArgs& d, uint32_t i, uint32_t& pl, uint32_t& r) {
     if (!d.trace_dir_major) return probe_sample(d, i, pl, r);
     r = i / d.np;
@@ -1490,6 +1493,7 @@ cudaError_t launch_probes(const SceneView& s, const ProbeArgs& d, uint32_t* out,
     if (cfg.phase_ev) cudaEventRecord(cfg.phase_ev[0], stream);
     LaunchConfig pcfg = cfg;
     pcfg.wide = cfg.wide && !cfg.primary_binary;
+    PP.d.trace_dir_major = d.trace_dir_major && (pcfg.wide || !use_walk(s, pcfg));
     cudaError_t e = use_walk(s, pcfg) ? launch_rays<false>(s, PP, n, counters + 0, err, stream, pcfg)
                                       : launch_general(s, PP, n, counters + 0, err, stream, pcfg);
     if (e != cudaSuccess) return e;
