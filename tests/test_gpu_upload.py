@@ -97,3 +97,26 @@ def test_bounds_of_the_vertices(native, oracle_mod):
             torch.cuda.synchronize()
             assert np.array_equal(hit.cpu().numpy().view(np.uint32), want.view(np.uint32))
             c.batch_destroy(batch)
+
+
+@pytest.mark.parametrize("tris", [3, 2000])
+def test_triangles_out_of_reach(native, oracle_mod, tris):
+    """The root's children are leaves without triangles; those of the image hang below them,
+    where no walk goes. Both ways of making the trees have to see that there is nothing to
+    make; one leaf with triangles beside an empty one makes them."""
+    from tim_raytracing_b200 import scenes
+    s = scenes.random_triangles(tris, tris)
+    img = native.build_bvh(s, max_leaf_size=1)
+    words = img.leaf_words()
+    zero = int(np.flatnonzero(words == 0)[0])   # a word that reads as a leaf of no triangles
+    tri = next(int(o) for o in img.nodes()[:, 3] if o != 0xFFFFFFFF and int(words[o]) & 0xFFF)
+    for offs in ((zero, zero), (tri, zero), (zero, tri)):
+        data = np.array(img.data, copy=True)
+        cut = dataclasses.replace(img, data=data)
+        nodes = cut.nodes()
+        left = int(nodes[0, 2]) & 0x3FFFFFFF
+        nodes[0, 2] = left | 0xC0000000
+        nodes[left, 3], nodes[left + 1, 3] = offs
+        with native.Context(0) as c:
+            sid = c.upload(cut, s)
+            _check(native, oracle_mod, c, sid, cut, s, tris)

@@ -177,9 +177,10 @@ __host__ __device__ __forceinline__ float divide(const Cover& l, const Cover& r,
 
 // An inner node's costs, and what they stand for: per number of slots k = 1 to 4, at bits
 // 4 (k - 1) and up, the left child's share of them and, above it, whether the node is
-// divided at all (it takes one slot otherwise). Made here once, so that the numbering of
-// the nodes reads one word a subtree: with both children's costs and three divisions for
-// each, a level of it took 13 to 23 us.
+// divided at all (it takes one slot otherwise); kHasTris unless no triangle is below. Made
+// here once, so that the numbering of the nodes reads one word a subtree: with both
+// children's costs and three divisions for each, a level of it took 13 to 23 us.
+constexpr uint32_t kHasTris = 1u << 16;
 struct NodeCost { float4 cost; uint32_t plan; };
 
 // Of an inner node with these children; area: its own box's.
@@ -193,7 +194,7 @@ __host__ __device__ __forceinline__ NodeCost cost_of(const In& in, const float4*
         if (r.f[0] == 0.0f) share[k] = k;   // no slot goes to a subtree without triangles (on the left none does)
     }
     const float single = area + d[4];
-    uint32_t plan = 0;
+    uint32_t plan = kHasTris;
     for (int k = 1; k <= 4; ++k) plan |= ((uint32_t)share[k] | (d[k] < single ? 8u : 0u)) << (4 * (k - 1));
     return {make_float4(least(single, d[1]), least(single, d[2]), least(single, d[3]), least(single, d[4])), plan};
 }
@@ -288,7 +289,7 @@ __host__ __device__ __forceinline__ void expand(const In& in, const uint32_t* pl
         if (b.k) st[sp++] = b;   // a subtree without triangles takes no slot
         if (a.k) st[sp++] = a;
     };
-    push(x, plan[x], 4, e);
+    if (plan[x] & kHasTris) push(x, plan[x], 4, e);   // only a root has none
     while (sp > 0) {
         const Sub s = st[--sp];
         if (!(s.id & kNidLeafBit)) {
@@ -358,8 +359,8 @@ __global__ void __launch_bounds__(128) k_four_level(In in, const uint32_t* plan,
 }
 
 // All levels of a small tree by one block, instead of a launch per level of the binary tree,
-// of which half are empty: the upload of 1,000 triangles 0.28 -> 0.25 ms, its second in a
-// context 0.25 -> 0.21.
+// of which half are empty: 55 us for 2,621 nodes, where a launch takes 8 to 12 us, an empty
+// one 4. With 3,300 inner nodes an upload took as long either way.
 constexpr uint32_t kSmallTree = 2048u, kSmallThreads = 512u;   // inner binary nodes
 __global__ void __launch_bounds__(kSmallThreads) k_four_small(In in, const uint32_t* plan, uint32_t* item, Box* item_e, uint2* base,
                                                     uint32_t cap, uint32_t depth, Ctl* ctl) {
@@ -665,7 +666,9 @@ TreeBuild::~TreeBuild() { dev_free(c, scratch); }   // waits for the kernels tha
 
 namespace {
 
-// Nodes up to which the host makes the trees.
+// Nodes up to which the host makes the trees: the whole upload by the host / by the kernels,
+// 63 nodes 0.043 / 0.13 ms, 651 0.084 / 0.12, 863 0.09 / 0.18, 2,015 0.196 / 0.169, 2,621
+// 0.28 / 0.185. The host takes 50 ns a node, the kernels' latencies 100 us and more.
 constexpr uint32_t kHostTree = 1536u;
 
 }  // namespace
