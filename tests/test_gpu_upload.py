@@ -116,6 +116,7 @@ def test_triangles_out_of_reach(native, oracle_mod, tris):
         nodes = cut.nodes()
         left = int(nodes[0, 2]) & 0x3FFFFFFF
         nodes[0, 2] = left | 0xC0000000
+        nodes[left:left + 2, 1] |= 0x80000000   # each other's sibling word says leaf too
         nodes[left, 3], nodes[left + 1, 3] = offs
         with native.Context(0) as c:
             sid = c.upload(cut, s)
