@@ -48,7 +48,8 @@
 // Measured (1080p frame of the 100K-triangle scene, 5.1M any-hit rays; 6.6M of the
 // 1279x719 frame with probe visibility): 1.07 -> 0.75 and 1.32 -> 0.94 ms against the
 // binary walk, with half the node visits (10.7 against 20.3 a ray) and 30 % fewer
-// instructions. The L1 binds it: 66 % of its data path's cycles, 57 % hits.
+// instructions (0.69 ms for the former since; four_stack.h has scenes of overlapping
+// boxes). The L1 binds it: 71 % of its data path's cycles, 61 % hits.
 #pragma once
 #include "common.cuh"
 #include "four_stack.h"

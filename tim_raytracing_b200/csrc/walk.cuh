@@ -372,7 +372,7 @@ static cudaError_t launch_walk_block(const SceneView& s, const Policy& P, uint32
 
 // One launch of k_walk, or one of a pair (of which the first may be given a share of the
 // GPU only). Stack words: a closest-hit ray leaves one child a level waiting, an any-hit
-// ray up to three slots, of which kAnyStack words are kept, a ray of the 8-wide form two
+// ray up to three slots or one word (four_words), a ray of the 8-wide form two
 // words a level; the end marker; and the word above the top, which a push writes whether
 // it keeps it or not.
 template <bool ANY, bool QUANT = false, class Policy>
